@@ -19,7 +19,10 @@
 // one fluid cell, so the scatter needs no atomics); velocity-face pulls and
 // the initial equilibrium accumulate the inflow gradient in FP64. States are
 // checkpointed every K calls during the forward run and recomputed segment by
-// segment (K = 1 stores every state and recomputes nothing).
+// segment, but for the last two segments, whose states the forward run leaves
+// in the sweep's buffers (K = 1 stores every state and recomputes nothing).
+// At 64^3, 200 calls, K = 20: 25 us a forward call and 72 us a call of the
+// sweep (49 and 140 before the pull classification and the kept segments).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -42,49 +45,91 @@ struct Geo {
     int nx, ny, nz;
     long long cells;
     int kind[6];  // per face: 1 periodic, 2 bounce-back, 4 velocity
-    const uint8_t* solid;
+    const uint2* links;  // pull classification of every cell (adj_links_kernel)
 };
 
-enum PullKind { kPullSlot = 0, kPullBounce = 1, kPullFace = 2 };
+// Pull classification of a fluid cell, built once per brick (the mask and the
+// face kinds never change): x holds one bit per direction whose source is
+// solid or outside a bounce-back face (plus kLinkSolid on solid cells), y one
+// bit per direction whose source is outside a velocity face.
+// The rules run 27 times per cell and launch otherwise: as branches they took
+// 32 of the forward launch's 50 us and about 70 of the reverse launch's 115
+// us at 64^3 (the initial call, which pulls nothing, ran in 18 and 43 us).
+// With the two words every population is one load or store at an address
+// formed by selects.
+constexpr unsigned kLinkSolid = 1u << 31;
 
-// Source of direction q for cell (x, y, z) (the brick step's pull rules:
-// periodic axes wrap; then the first out-of-range axis in the order x-, x+,
-// y-, y+, z-, z+ names the face).
-__host__ __device__ __forceinline__ int pull_source(const Geo& G, int x, int y, int z, int q, long long& src) {
-    int s[3] = {x - q_cx(q), y - q_cy(q), z - q_cz(q)};
+__global__ void adj_links_kernel(Geo G, const uint8_t* __restrict__ solid, uint2* __restrict__ links) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= G.cells) return;
+    unsigned bounce = solid[i] ? kLinkSolid : 0u, inflow = 0u;
+    int c[3];
+    cell_xyz32(i, G.ny, G.nz, c[0], c[1], c[2]);
     const int n[3] = {G.nx, G.ny, G.nz};
-    int face = -1;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (s[a] < 0 || s[a] >= n[a]) {
+    for (int q = 0; q < 27; ++q) {
+        // periodic axes wrap; then the first out-of-range axis in the order
+        // x-, x+, y-, y+, z-, z+ names the face
+        int s[3] = {c[0] - q_cx(q), c[1] - q_cy(q), c[2] - q_cz(q)};
+        int face = -1;
+        for (int a = 0; a < 3; ++a) {
+            if (s[a] >= 0 && s[a] < n[a]) continue;
             const int fid = 2 * a + (s[a] < 0 ? 0 : 1);
-            if (G.kind[fid] == kHydroPeriodic) {
-                s[a] = s[a] < 0 ? s[a] + n[a] : s[a] - n[a];
-            } else if (face < 0) {
-                face = fid;
-            }
+            if (G.kind[fid] == kHydroPeriodic) s[a] = s[a] < 0 ? s[a] + n[a] : s[a] - n[a];
+            else if (face < 0) face = fid;
+        }
+        if (face >= 0) {
+            if (G.kind[face] == kHydroVelocity) inflow |= 1u << q;
+            else bounce |= 1u << q;
+        } else if (solid[((long long)s[0] * G.ny + s[1]) * G.nz + s[2]]) {
+            bounce |= 1u << q;
         }
     }
-    if (face >= 0) return G.kind[face] == kHydroVelocity ? kPullFace : kPullBounce;
-    src = ((long long)s[0] * G.ny + s[1]) * G.nz + s[2];
-    return G.solid[src] ? kPullBounce : kPullSlot;
+    links[i] = make_uint2(bounce, inflow);
+}
+
+// Cell index of the neighbour along -c_q: one term per axis. A coordinate
+// that leaves the brick wraps; a link that leaves by a face that is not
+// periodic never uses the index.
+struct Neighbours {
+    unsigned X[3], Y[3], Z[3];
+    __device__ __forceinline__ Neighbours(const Geo& G, int x, int y, int z) {
+        const unsigned row = (unsigned)G.nz, slab = (unsigned)G.ny * row;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int sx = x + k - 1, sy = y + k - 1, sz = z + k - 1;
+            X[k] = (unsigned)(sx < 0 ? sx + G.nx : (sx >= G.nx ? sx - G.nx : sx)) * slab;
+            Y[k] = (unsigned)(sy < 0 ? sy + G.ny : (sy >= G.ny ? sy - G.ny : sy)) * row;
+            Z[k] = (unsigned)(sz < 0 ? sz + G.nz : (sz >= G.nz ? sz - G.nz : sz));
+        }
+    }
+    __device__ __forceinline__ unsigned source(int q) const { return X[1 - q_cx(q)] + Y[1 - q_cy(q)] + Z[1 - q_cz(q)]; }
+};
+
+// The population a pull of direction q reads: the source cell's, or after a
+// bounce the cell's own opposite one.
+// I: unsigned where every slot index of a state fits 32 bits, else 64 bits.
+template <class I>
+__device__ __forceinline__ I link_slot(const Geo& G, const Neighbours& nb, unsigned own, unsigned i, int q) {
+    const I bounced = (I)q_opp(q) * (I)G.cells + i, pulled = (I)q * (I)G.cells + nb.source(q);
+    return (own >> q) & 1u ? bounced : pulled;
+}
+
+// Streamed populations of a fluid cell.
+template <class I, class T>
+__device__ __forceinline__ void pull_cell(const Geo& G, const T* __restrict__ s, long long i, const Neighbours& nb, uint2 w,
+                                          const T (&uin)[3], T (&p)[27]) {
+    const unsigned own = w.x | w.y;
+#pragma unroll
+    for (int q = 0; q < 27; ++q) p[q] = s[link_slot<I>(G, nb, own, (unsigned)i, q)];
+    if (w.y) {
+#pragma unroll
+        for (int q = 0; q < 27; ++q)
+            if ((w.y >> q) & 1u) p[q] = feq_t<T>(q, T(1), uin[0], uin[1], uin[2]);
+    }
 }
 
 __device__ __forceinline__ void cell_xyz(const Geo& G, long long i, int& x, int& y, int& z) {
     cell_xyz32(i, G.ny, G.nz, x, y, z);
-}
-
-template <class T>
-__device__ __forceinline__ void pull_cell(const Geo& G, const T* __restrict__ s, long long i, int x, int y, int z,
-                                          const T (&uin)[3], T (&p)[27]) {
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        long long src = 0;
-        const int k = pull_source(G, x, y, z, q, src);
-        p[q] = k == kPullSlot ? s[(long long)q * G.cells + src]
-             : k == kPullBounce ? s[(long long)q_opp(q) * G.cells + i]
-                                : feq_t<T>(q, T(1), uin[0], uin[1], uin[2]);
-    }
 }
 
 template <class T>
@@ -110,14 +155,15 @@ __device__ __forceinline__ void cell_force(const StepArgs<T>& A, long long i, T&
 }
 
 // One forward call: init (kInit, collide the equilibrium) or pull + collide.
-template <class T, bool kInit>
+template <class T, bool kInit, class I>
 __global__ void __launch_bounds__(128) adj_step_kernel(StepArgs<T> A) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= A.G.cells) return;
     T* __restrict__ dst = A.dst;
-    if (A.G.solid[i]) {
+    const uint2 w = A.G.links[i];
+    if (w.x & kLinkSolid) {
 #pragma unroll
-        for (int q = 0; q < 27; ++q) dst[(long long)q * A.G.cells + i] = wq<T>(q);
+        for (int q = 0; q < 27; ++q) dst[(I)q * (I)A.G.cells + (unsigned)i] = wq<T>(q);
         return;
     }
     T p[27];
@@ -127,7 +173,7 @@ __global__ void __launch_bounds__(128) adj_step_kernel(StepArgs<T> A) {
     } else {
         int x, y, z;
         cell_xyz(A.G, i, x, y, z);
-        pull_cell<T>(A.G, A.src, i, x, y, z, A.uin, p);
+        pull_cell<I>(A.G, A.src, i, Neighbours(A.G, x, y, z), w, A.uin, p);
     }
     T t, fx, fy, fz;
     cell_force(A, i, t, fx, fy, fz);
@@ -135,7 +181,7 @@ __global__ void __launch_bounds__(128) adj_step_kernel(StepArgs<T> A) {
     CollideTape<T> tape;
     collide_fwd<T>(p, A.cp, t, fx, fy, fz, fo, tape);
 #pragma unroll
-    for (int q = 0; q < 27; ++q) dst[(long long)q * A.G.cells + i] = fo[q];
+    for (int q = 0; q < 27; ++q) dst[(I)q * (I)A.G.cells + (unsigned)i] = fo[q];
 }
 
 // Probe velocities of P(s) and the loss sum (FP64).
@@ -151,7 +197,7 @@ __global__ void adj_probe_kernel(Geo G, const T* __restrict__ s, T ux_in, T uy_i
     const T uin[3] = {ux_in, uy_in, uz_in};
     T p[27], u[3], rc;
     bool rf;
-    pull_cell<T>(G, s, i, x, y, z, uin, p);
+    pull_cell<unsigned long long>(G, s, i, Neighbours(G, x, y, z), G.links[i], uin, p);
     probe_velocity<T>(p, u, rc, rf);
     double l = 0.0;
 #pragma unroll
@@ -171,25 +217,27 @@ __global__ void adj_probe_kernel(Geo G, const T* __restrict__ s, T ux_in, T uy_i
 // population, so its adjoint is zero, written here. With kAccumulate false
 // the launch therefore writes every fluid slot of lam_prev exactly once and
 // needs no clearing pass (solid cells' slots are never read).
-template <bool kAccumulate>
-__device__ __forceinline__ void scatter(const Geo& G, long long i, int x, int y, int z, const float (&lam)[27],
+template <bool kAccumulate, class I>
+__device__ __forceinline__ void scatter(const Geo& G, long long i, const Neighbours& nb, uint2 w, const float (&lam)[27],
                                         const float (&uin)[3], float* __restrict__ lam_prev, double (&du)[3]) {
+    const unsigned own = w.x | w.y;
+    if (w.y) {
 #pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        long long src = 0;
-        const int k = pull_source(G, x, y, z, q, src);
-        if (k == kPullFace) {
+        for (int q = 0; q < 27; ++q) {
+            if (!((w.y >> q) & 1u)) continue;
             float d[3];
             dfeq_du<float>(q, 1.0f, uin[0], uin[1], uin[2], d);
             du[0] += (double)lam[q] * d[0];
             du[1] += (double)lam[q] * d[1];
             du[2] += (double)lam[q] * d[2];
-            if (!kAccumulate) lam_prev[(long long)q_opp(q) * G.cells + i] = 0.0f;
-            continue;
         }
-        float* slot = k == kPullSlot ? lam_prev + (long long)q * G.cells + src : lam_prev + (long long)q_opp(q) * G.cells + i;
-        if (kAccumulate) *slot += lam[q];
-        else *slot = lam[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        float* slot = lam_prev + link_slot<I>(G, nb, own, (unsigned)i, q);
+        const bool inflow = (w.y >> q) & 1u;
+        if (!kAccumulate) *slot = inflow ? 0.0f : lam[q];
+        else if (!inflow) *slot += lam[q];
     }
 }
 
@@ -217,52 +265,72 @@ __device__ __forceinline__ void add_du(double (&du)[3], double* __restrict__ du_
     }
 }
 
-// lambda_N at the probe cells: dL/du through the probe observable, scattered
-// (one thread, probes in order: probes may share slots).
+// lambda_N at the probe cells: dL/du through the probe observable, scattered.
+// One warp per probe: the pulls of different cells read different slots, so
+// only probes of one cell share slots; the first of them adds all of its
+// cell's probes in order, the others do nothing. Inflow-gradient parts go to
+// the probe's own entry of du_probe. (As one thread over all probes, each
+// waiting for the last one's loads, the 64 probes of a 64^3 brick took 1056
+// us.)
 __global__ void adj_seed_kernel(Geo G, const float* __restrict__ s, float ux_in, float uy_in, float uz_in, int nprobe,
                                 const long long* __restrict__ cells, const float* __restrict__ target,
-                                float* __restrict__ lam, double* __restrict__ du_slot) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+                                float* __restrict__ lam, double* __restrict__ du_probe) {
+    const int first = blockIdx.x;
+    const long long i = cells[first];
+    bool earlier = false;
+    for (int k = threadIdx.x; k < first; k += 32) earlier |= cells[k] == i;
     double du[3] = {0.0, 0.0, 0.0};
-    for (int k = 0; k < nprobe; ++k) {
-        const long long i = cells[k];
+    if (!__any_sync(0xffffffffu, earlier) && threadIdx.x == 0) {
         int x, y, z;
         cell_xyz(G, i, x, y, z);
         const float uin[3] = {ux_in, uy_in, uz_in};
+        const Neighbours nb(G, x, y, z);
+        const uint2 w = G.links[i];
         float p[27], u[3], rc;
         bool rf;
-        pull_cell<float>(G, s, i, x, y, z, uin, p);
+        pull_cell<unsigned long long>(G, s, i, nb, w, uin, p);
         probe_velocity<float>(p, u, rc, rf);
-        const float lu[3] = {2.0f * (u[0] - target[3 * k]), 2.0f * (u[1] - target[3 * k + 1]), 2.0f * (u[2] - target[3 * k + 2])};
-        float lp[27];
-        probe_velocity_vjp<float>(u, rc, rf, lu, lp);
-        scatter<true>(G, i, x, y, z, lp, uin, lam, du);
+        for (int k = first; k < nprobe; ++k) {
+            if (cells[k] != i) continue;
+            const float lu[3] = {2.0f * (u[0] - target[3 * k]), 2.0f * (u[1] - target[3 * k + 1]),
+                                 2.0f * (u[2] - target[3 * k + 2])};
+            float lp[27];
+            probe_velocity_vjp<float>(u, rc, rf, lu, lp);
+            scatter<true, unsigned long long>(G, i, nb, w, lp, uin, lam, du);
+        }
     }
-    du_slot[0] = du[0];
-    du_slot[1] = du[1];
-    du_slot[2] = du[2];
+    if (threadIdx.x == 0)
+        for (int a = 0; a < 3; ++a) du_probe[3 * first + a] = du[a];
 }
 
 // One reverse call: lambda_n (cell-local read) -> lambda_{n-1} (scatter),
 // body-force gradient of the cell, inflow gradient.
-#ifndef AERO_ADJ_REV_MIN_BLOCKS
-#define AERO_ADJ_REV_MIN_BLOCKS 5
-#endif
-template <bool kInit>
-__global__ void __launch_bounds__(128, AERO_ADJ_REV_MIN_BLOCKS) adj_reverse_kernel(StepArgs<float> A, const float* __restrict__ lam_n,
+// Latency-bound (long scoreboard) at 20 warps per SM, the most that its
+// registers allow. Of the block sizes that keep 20 warps, 320 threads measured
+// best where the grid fills the chip (64^3, sweep per call: 72 us against 74
+// of 128, 78 of 64 and 72 of 640 threads); below about one and a half waves
+// the smaller blocks spread better (48^3: 36.5 against 33.9 us, 56^3: 44.9
+// against 46.2), so rev_threads_for draws the line there.
+constexpr int kRevThreads = 320, kRevThreadsSmall = 128;
+constexpr long long kRevWaveCells = 148LL * 2 * kRevThreads;
+int rev_threads_for(long long cells) { return 2 * cells >= 3 * kRevWaveCells ? kRevThreads : kRevThreadsSmall; }
+template <bool kInit, class I>
+__global__ void __launch_bounds__(kRevThreads, 2) adj_reverse_kernel(StepArgs<float> A, const float* __restrict__ lam_n,
                                                           float* __restrict__ lam_prev, double* __restrict__ grad_f,
                                                           double* __restrict__ du_part) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double du[3] = {0.0, 0.0, 0.0};
-    if (i < A.G.cells && !A.G.solid[i]) {
+    const uint2 w = i < A.G.cells ? A.G.links[i] : make_uint2(kLinkSolid, 0u);
+    if (!(w.x & kLinkSolid)) {
         int x, y, z;
         cell_xyz(A.G, i, x, y, z);
+        const Neighbours nb(A.G, x, y, z);
         float p[27];
         if (kInit) {
 #pragma unroll
             for (int q = 0; q < 27; ++q) p[q] = feq_t<float>(q, 1.0f, A.uin[0], A.uin[1], A.uin[2]);
         } else {
-            pull_cell<float>(A.G, A.src, i, x, y, z, A.uin, p);
+            pull_cell<I>(A.G, A.src, i, nb, w, A.uin, p);
         }
         float t, fx, fy, fz;
         cell_force(A, i, t, fx, fy, fz);
@@ -273,9 +341,11 @@ __global__ void __launch_bounds__(128, AERO_ADJ_REV_MIN_BLOCKS) adj_reverse_kern
 #pragma unroll
         for (int q = 0; q < 27; ++q) lo[q] = lam_n[(long long)q * A.G.cells + i];
         collide_vjp<float>(tape, A.cp, lo, li, lf);
-        grad_f[i] += (double)lf[0];
-        grad_f[A.G.cells + i] += (double)lf[1];
-        grad_f[2 * A.G.cells + i] += (double)lf[2];
+        // one thread per entry, one launch after the other: the sums keep their
+        // order, and an addition in L2 needs no load to wait for
+        atomicAdd(grad_f + i, (double)lf[0]);
+        atomicAdd(grad_f + A.G.cells + i, (double)lf[1]);
+        atomicAdd(grad_f + 2 * A.G.cells + i, (double)lf[2]);
         if (kInit) {
 #pragma unroll
             for (int q = 0; q < 27; ++q) {
@@ -286,7 +356,7 @@ __global__ void __launch_bounds__(128, AERO_ADJ_REV_MIN_BLOCKS) adj_reverse_kern
                 du[2] += (double)li[q] * d[2];
             }
         } else {
-            scatter<false>(A.G, i, x, y, z, li, A.uin, lam_prev, du);
+            scatter<false, I>(A.G, i, nb, w, li, A.uin, lam_prev, du);
         }
     }
     add_du(du, du_part);
@@ -299,19 +369,23 @@ struct Brick {
     CollideParams cp{};
     long long cells = 0;
     size_t state_elems = 0;
+    void* block = nullptr;     // one allocation: the arrays below up to the inflow-gradient parts
     uint8_t* solid = nullptr;
     float* temperature = nullptr;
     float* force = nullptr;
     float* st[2] = {nullptr, nullptr};
     double* st64[2] = {nullptr, nullptr};
+    void* sweep = nullptr;     // one block: the checkpoint and segment states
     std::vector<float*> ckpt;  // ckpt[j] = s_{jK} for j >= 1 (index 0 unused)
-    std::vector<float*> seg;   // two sets of K - 1 recomputed segment states
+    std::vector<float*> seg;   // two sets of K - 1 segment states
     cudaStream_t side = nullptr;  // recomputation stream (overlaps the reverse launches)
     float* lam[2] = {nullptr, nullptr};
     double* grad_f = nullptr;
     double* probe_loss = nullptr;  // per probe
-    double* du_part = nullptr;     // 3 x (reverse blocks + 1): inflow-gradient parts, the last slot from the seed
-    int rev_blocks = 0;
+    double* du_part = nullptr;     // 3 x reverse blocks: inflow-gradient parts of the reverse launches
+    double* du_probe = nullptr;    // 3 x probes: those of the seed
+    uint2* links = nullptr;        // pull classification
+    int rev_blocks = 0, rev_threads = 0;
     int nprobe = 0;
     long long* probe_cells = nullptr;
     float* probe_target = nullptr;
@@ -320,13 +394,8 @@ struct Brick {
     int fwd_steps = 0, rev_steps = 0;
 
     ~Brick() {
-        for (void* p : {(void*)solid, (void*)temperature, (void*)force, (void*)st[0], (void*)st[1], (void*)st64[0],
-                        (void*)st64[1], (void*)lam[0], (void*)lam[1], (void*)grad_f, (void*)probe_loss, (void*)du_part, (void*)probe_cells,
+        for (void* p : {block, sweep, (void*)st64[0], (void*)st64[1], (void*)probe_loss, (void*)du_probe, (void*)probe_cells,
                         (void*)probe_target, (void*)probe_u})
-            if (p) cudaFree(p);
-        for (float* p : ckpt)
-            if (p) cudaFree(p);
-        for (float* p : seg)
             if (p) cudaFree(p);
         if (side) cudaStreamDestroy(side);
     }
@@ -376,13 +445,20 @@ StepArgs<T> step_args(const Brick& b, const float* inflow, const T* src, T* dst)
     return a;
 }
 
+size_t aligned(size_t bytes) { return (bytes + 255) / 256 * 256; }
+
+// Slot indices of a state fit 32 bits (one address operation less per load).
+bool narrow(const Brick& b) { return b.state_elems < (1ull << 32); }
+
 unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 template <class T>
 bool launch_step(const Brick& b, const float* inflow, bool init, const T* src, T* dst, cudaStream_t s) {
     const StepArgs<T> a = step_args<T>(b, inflow, src, dst);
-    if (init) adj_step_kernel<T, true><<<blocks_for(b.cells, 128), 128, 0, s>>>(a);
-    else adj_step_kernel<T, false><<<blocks_for(b.cells, 128), 128, 0, s>>>(a);
+    const unsigned blocks = blocks_for(b.cells, 128);
+    if (init) adj_step_kernel<T, true, unsigned long long><<<blocks, 128, 0, s>>>(a);
+    else if (narrow(b)) adj_step_kernel<T, false, unsigned><<<blocks, 128, 0, s>>>(a);
+    else adj_step_kernel<T, false, unsigned long long><<<blocks, 128, 0, s>>>(a);
     count_launch();
     return adj_ok(cudaGetLastError(), "adjoint forward step");
 }
@@ -454,20 +530,38 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_adjoint_create(const AeroLbmB200AdjointCo
     b->state_elems = (size_t)b->cells * 27;
     b->cp = params_of(*cfg);
     const size_t n = (size_t)b->cells;
-    bool ok = adj_ok(cudaMalloc(&b->solid, n), "adjoint alloc") &&
-              adj_ok(cudaMalloc(&b->force, 3 * n * sizeof(float)), "adjoint alloc") &&
-              adj_ok(cudaMalloc(&b->st[0], b->state_elems * sizeof(float)), "adjoint alloc") &&
-              adj_ok(cudaMalloc(&b->st[1], b->state_elems * sizeof(float)), "adjoint alloc") &&
-              adj_ok(cudaMalloc(&b->lam[0], b->state_elems * sizeof(float)), "adjoint alloc") &&
-              adj_ok(cudaMalloc(&b->lam[1], b->state_elems * sizeof(float)), "adjoint alloc") &&
-              adj_ok(cudaMalloc(&b->grad_f, 3 * n * sizeof(double)), "adjoint alloc") &&
-              adj_ok(cudaMalloc(&b->du_part, 3 * ((size_t)blocks_for(b->cells, 128) + 1) * sizeof(double)), "adjoint alloc");
-    b->rev_blocks = (int)blocks_for(b->cells, 128);
+    b->rev_threads = rev_threads_for(b->cells);
+    b->rev_blocks = (int)blocks_for(b->cells, b->rev_threads);
+    // the brick's arrays are slices of one block (ten allocations otherwise)
+    struct Slice {
+        void** to;
+        size_t bytes;
+    };
+    const std::vector<Slice> slices = {{(void**)&b->st[0], b->state_elems * sizeof(float)},
+                                       {(void**)&b->st[1], b->state_elems * sizeof(float)},
+                                       {(void**)&b->lam[0], b->state_elems * sizeof(float)},
+                                       {(void**)&b->lam[1], b->state_elems * sizeof(float)},
+                                       {(void**)&b->grad_f, 3 * n * sizeof(double)},
+                                       {(void**)&b->du_part, 3 * (size_t)b->rev_blocks * sizeof(double)},
+                                       {(void**)&b->links, n * sizeof(uint2)},
+                                       {(void**)&b->force, 3 * n * sizeof(float)},
+                                       {(void**)&b->temperature, temperature ? n * sizeof(float) : 0},
+                                       {(void**)&b->solid, n}};
+    size_t total = 0;
+    for (const Slice& x : slices) total += aligned(x.bytes);
+    bool ok = adj_ok(cudaMalloc(&b->block, total), "adjoint alloc");
+    char* next = static_cast<char*>(b->block);
+    for (const Slice& x : slices) {
+        if (!ok || !x.bytes) continue;
+        *x.to = next;
+        next += aligned(x.bytes);
+    }
+    const cudaStream_t s = current_stream();
     if (ok && temperature)
-        ok = adj_ok(cudaMalloc(&b->temperature, n * sizeof(float)), "adjoint alloc") &&
-             adj_ok(cudaMemcpy(b->temperature, temperature, n * sizeof(float), cudaMemcpyHostToDevice), "temperature upload");
-    if (ok) ok = adj_ok(cudaMemcpy(b->solid, obstacle, n, cudaMemcpyHostToDevice), "mask upload");
+        ok = adj_ok(cudaMemcpyAsync(b->temperature, temperature, n * sizeof(float), cudaMemcpyHostToDevice, s), "temperature upload");
+    if (ok) ok = adj_ok(cudaMemcpyAsync(b->solid, obstacle, n, cudaMemcpyHostToDevice, s), "mask upload");
     if (!ok) {
+        cudaStreamSynchronize(s);
         delete b;
         return 0;
     }
@@ -476,7 +570,13 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_adjoint_create(const AeroLbmB200AdjointCo
     b->geo.nz = cfg->nz;
     b->geo.cells = b->cells;
     for (int f = 0; f < 6; ++f) b->geo.kind[f] = cfg->face_kind[f];
-    b->geo.solid = b->solid;
+    b->geo.links = b->links;
+    adj_links_kernel<<<blocks_for(b->cells, 256), 256, 0, s>>>(b->geo, b->solid, b->links);
+    count_launch();
+    if (!adj_ok(cudaGetLastError(), "adjoint links") || !adj_ok(cudaStreamSynchronize(s), "adjoint links")) {
+        delete b;
+        return 0;
+    }
     const long long h = g_next_adj++;
     g_adj[h] = b;
     *out_handle = h;
@@ -501,9 +601,10 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_adjoint_set_probes(long long handle, int 
         }
         c[k] = cells[k];
     }
-    for (void* p : {(void*)b->probe_cells, (void*)b->probe_target, (void*)b->probe_u, (void*)b->probe_loss})
+    for (void* p : {(void*)b->probe_cells, (void*)b->probe_target, (void*)b->probe_u, (void*)b->probe_loss, (void*)b->du_probe})
         if (p) cudaFree(p);
     b->probe_cells = nullptr;
+    b->du_probe = nullptr;
     b->probe_target = b->probe_u = nullptr;
     b->probe_loss = nullptr;
     b->nprobe = 0;
@@ -511,6 +612,7 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_adjoint_set_probes(long long handle, int 
         !adj_ok(cudaMalloc(&b->probe_target, 3 * count * sizeof(float)), "probe alloc") ||
         !adj_ok(cudaMalloc(&b->probe_u, 3 * count * sizeof(float)), "probe alloc") ||
         !adj_ok(cudaMalloc(&b->probe_loss, count * sizeof(double)), "probe alloc") ||
+        !adj_ok(cudaMalloc(&b->du_probe, 3 * (size_t)count * sizeof(double)), "probe alloc") ||
         !adj_ok(cudaMemcpy(b->probe_cells, c.data(), count * sizeof(long long), cudaMemcpyHostToDevice), "probe upload") ||
         !adj_ok(cudaMemcpy(b->probe_target, targets, 3 * count * sizeof(float), cudaMemcpyHostToDevice), "probe upload"))
         return 0;
@@ -589,53 +691,66 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_adjoint_gradient(long long handle, const 
     const Geo G = b->geo;
     const size_t bytes = b->state_elems * sizeof(float);
     // checkpoint and segment states, allocated at the first gradient call
-    // (forward-only use needs neither)
-    if (b->ckpt.empty()) {
+    // (forward-only use needs neither) as slices of one block: 47 allocations
+    // of a 64^3 brick's 28 MB took most of that call
+    if (!b->sweep) {
         const int segments = (N + K - 1) / K;
-        b->ckpt.assign(segments, nullptr);
-        b->seg.assign(2 * std::max(0, K - 1), nullptr);
-        bool got = true;
-        for (int j = 1; got && j < segments; ++j) got = adj_ok(cudaMalloc(&b->ckpt[j], bytes), "checkpoint alloc");
-        for (size_t j = 0; got && j < b->seg.size(); ++j) got = adj_ok(cudaMalloc(&b->seg[j], bytes), "segment alloc");
-        if (got && !b->side) got = adj_ok(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking), "side stream");
-        if (!got) {
-            for (float* p : b->ckpt)
-                if (p) cudaFree(p);
-            for (float* p : b->seg)
-                if (p) cudaFree(p);
-            b->ckpt.clear();
-            b->seg.clear();
+        const size_t slices = (size_t)segments - 1 + 2 * (size_t)std::max(0, K - 1);
+        const size_t slice = aligned(bytes);
+        if (!b->side && !adj_ok(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking), "side stream")) return 0;
+        if (!adj_ok(cudaMalloc(&b->sweep, std::max<size_t>(1, slices) * slice), "checkpoint and segment alloc")) {
+            b->sweep = nullptr;
             return 0;
         }
+        char* next = static_cast<char*>(b->sweep);
+        auto take = [&] {
+            float* p = reinterpret_cast<float*>(next);
+            next += slice;
+            return p;
+        };
+        b->ckpt.assign(segments, nullptr);
+        for (int j = 1; j < segments; ++j) b->ckpt[j] = take();
+        b->seg.clear();
+        for (int j = 0; j < 2 * std::max(0, K - 1); ++j) b->seg.push_back(take());
     }
     cudaEvent_t ev[6];
     for (auto& e : ev) cudaEventCreate(&e);
-    const size_t du_bytes = 3 * ((size_t)b->rev_blocks + 1) * sizeof(double);
+    const size_t du_bytes = 3 * (size_t)b->rev_blocks * sizeof(double);
     bool ok = upload_force(*b, force_soa, s) && adj_ok(cudaMemsetAsync(b->du_part, 0, du_bytes, s), "clear") &&
               adj_ok(cudaMemsetAsync(b->grad_f, 0, 3 * b->cells * sizeof(double), s), "clear");
-    // forward with checkpoints s_{jK}
+    // forward run. A checkpoint is written by its own launch, and so are the
+    // states of the last two segments: their two buffer sets are idle until
+    // the sweep reverses those segments, so these need no recomputation.
+    const int segments = (N + K - 1) / K;
+    const int per = std::max(0, K - 1);
+    auto kept = [&](int n) -> float* {  // where s_n stays for the sweep (null: nowhere)
+        const int j = n / K, m = n - j * K;
+        if (n >= N) return nullptr;
+        if (m == 0) return b->ckpt[j];
+        return j >= segments - 2 ? b->seg[(size_t)(segments - 1 - j) * per + m - 1] : nullptr;
+    };
     cudaEventRecord(ev[0], s);
+    float* state = kept(1) ? kept(1) : b->st[0];
     int cur = 0;
-    ok = ok && launch_step<float>(*b, inflow, true, nullptr, b->st[0], s);
-    if (ok && K == 1 && N >= 2) ok = adj_ok(cudaMemcpyAsync(b->ckpt[1], b->st[0], bytes, cudaMemcpyDeviceToDevice, s), "ckpt");
+    ok = ok && launch_step<float>(*b, inflow, true, nullptr, state, s);
     for (int n = 2; ok && n <= N; ++n) {
-        ok = launch_step<float>(*b, inflow, false, b->st[cur], b->st[cur ^ 1], s);
-        cur ^= 1;
-        if (ok && n % K == 0 && n < N)
-            ok = adj_ok(cudaMemcpyAsync(b->ckpt[n / K], b->st[cur], bytes, cudaMemcpyDeviceToDevice, s), "checkpoint");
+        float* dst = kept(n);
+        if (!dst) dst = b->st[cur ^= 1];
+        ok = launch_step<float>(*b, inflow, false, state, dst, s);
+        state = dst;
     }
     cudaEventRecord(ev[1], s);
     // loss and the seed of lambda_N
     if (ok) {
-        adj_probe_kernel<float><<<blocks_for(b->nprobe, 64), 64, 0, s>>>(G, b->st[cur], inflow[0], inflow[1], inflow[2],
+        adj_probe_kernel<float><<<blocks_for(b->nprobe, 64), 64, 0, s>>>(G, state, inflow[0], inflow[1], inflow[2],
                                                                           b->nprobe, b->probe_cells, b->probe_target,
                                                                           b->probe_u, b->probe_loss);
         count_launch();
         ok = adj_ok(cudaMemsetAsync(b->lam[0], 0, bytes, s), "lambda clear");
     }
     if (ok) {
-        adj_seed_kernel<<<1, 32, 0, s>>>(G, b->st[cur], inflow[0], inflow[1], inflow[2], b->nprobe, b->probe_cells,
-                                          b->probe_target, b->lam[0], b->du_part + 3 * (size_t)b->rev_blocks);
+        adj_seed_kernel<<<b->nprobe, 32, 0, s>>>(G, state, inflow[0], inflow[1], inflow[2], b->nprobe, b->probe_cells,
+                                                 b->probe_target, b->lam[0], b->du_probe);
         count_launch();
         ok = adj_ok(cudaGetLastError(), "seed kernel");
     }
@@ -646,8 +761,6 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_adjoint_gradient(long long handle, const 
     // recomputation reads only checkpoint j - 1, so the two run side by side.
     int lc = 0;
     double rec_ms = 0.0, rev_ms = 0.0;
-    const int segments = (N + K - 1) / K;
-    const int per = std::max(0, K - 1);
     cudaStream_t s2 = b->side;
     std::vector<cudaEvent_t> evw(segments), evr(segments), eve(segments);  // on s: before / after the wait, after the reverse
     cudaEvent_t rec_done[2], rev_done[2], fwd_done;
@@ -677,27 +790,26 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_adjoint_gradient(long long handle, const 
         }
         return adj_ok(cudaEventRecord(rec_done[set], s2), "segment done");
     };
-    if (ok && segments > 0) ok = recompute(segments - 1, 0);
     for (int j = segments - 1, idx = 0; ok && j >= 0; --j, ++idx) {
         const int set = idx % 2;
-        if (j > 0) ok = recompute(j - 1, set ^ 1);
+        if (j > 0 && j - 1 < segments - 2) ok = recompute(j - 1, set ^ 1);
         const int first = j * K + 1, last = std::min((j + 1) * K, N);
         // states[m] = s_{jK + m} for m = 1 .. last - first (s_{jK} = ckpt[j])
         std::vector<const float*> states(last - first + 1, nullptr);
         states[0] = j > 0 ? b->ckpt[j] : nullptr;
         for (int m = 1; m <= last - first; ++m) states[m] = b->seg[(size_t)set * per + m - 1];
-        ok = ok && adj_ok(cudaEventRecord(evw[idx], s), "sweep event") && adj_ok(cudaStreamWaitEvent(s, rec_done[set], 0), "segment wait") &&
+        ok = ok && adj_ok(cudaEventRecord(evw[idx], s), "sweep event") && (j >= segments - 2 || adj_ok(cudaStreamWaitEvent(s, rec_done[set], 0), "segment wait")) &&
              adj_ok(cudaEventRecord(evr[idx], s), "sweep event");
         for (int n = last; ok && n >= first; --n) {
             const int m = n - first;  // input state of call n is states[m]
             StepArgs<float> a = step_args<float>(*b, inflow, states[m], nullptr);
             // the reverse launch writes every fluid slot of lam[lc ^ 1] (scatter)
-            if (n == 1)
-                adj_reverse_kernel<true><<<blocks_for(b->cells, 128), 128, 0, s>>>(a, b->lam[lc], b->lam[lc ^ 1], b->grad_f,
-                                                                                   b->du_part);
-            else
-                adj_reverse_kernel<false><<<blocks_for(b->cells, 128), 128, 0, s>>>(a, b->lam[lc], b->lam[lc ^ 1], b->grad_f,
-                                                                                    b->du_part);
+            const unsigned blocks = b->rev_blocks;
+            const int threads = b->rev_threads;
+            float *lam = b->lam[lc], *prev = b->lam[lc ^ 1];
+            if (n == 1) adj_reverse_kernel<true, unsigned long long><<<blocks, threads, 0, s>>>(a, lam, prev, b->grad_f, b->du_part);
+            else if (narrow(*b)) adj_reverse_kernel<false, unsigned><<<blocks, threads, 0, s>>>(a, lam, prev, b->grad_f, b->du_part);
+            else adj_reverse_kernel<false, unsigned long long><<<blocks, threads, 0, s>>>(a, lam, prev, b->grad_f, b->du_part);
             count_launch();
             ok = adj_ok(cudaGetLastError(), "reverse kernel");
             lc ^= 1;
@@ -720,10 +832,12 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_adjoint_gradient(long long handle, const 
         cudaEventDestroy(rev_done[k]);
     }
     cudaEventDestroy(fwd_done);
-    std::vector<double> pl(b->nprobe), du(3 * ((size_t)b->rev_blocks + 1));
+    std::vector<double> pl(b->nprobe), du(3 * ((size_t)b->rev_blocks + b->nprobe));
     if (ok) ok = adj_ok(cudaMemcpyAsync(pl.data(), b->probe_loss, b->nprobe * sizeof(double), cudaMemcpyDeviceToHost, s),
                         "loss read") &&
-                 adj_ok(cudaMemcpyAsync(du.data(), b->du_part, du_bytes, cudaMemcpyDeviceToHost, s), "gradient read");
+                 adj_ok(cudaMemcpyAsync(du.data(), b->du_part, du_bytes, cudaMemcpyDeviceToHost, s), "gradient read") &&
+                 adj_ok(cudaMemcpyAsync(du.data() + 3 * (size_t)b->rev_blocks, b->du_probe, 3 * (size_t)b->nprobe * sizeof(double),
+                                        cudaMemcpyDeviceToHost, s), "gradient read");
     if (ok && out_grad_force)
         ok = adj_ok(cudaMemcpyAsync(out_grad_force, b->grad_f, 3 * b->cells * sizeof(double), cudaMemcpyDeviceToHost, s),
                     "gradient read");

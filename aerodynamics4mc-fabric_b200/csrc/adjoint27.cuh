@@ -56,6 +56,32 @@ __host__ __device__ __forceinline__ void dfeq_du(int q, T rho, T ux, T uy, T uz,
     d[2] = k * (T(3) * cz + cu * T(3) * cz - T(3) * uz);
 }
 
+// c_q . (x, y, z) over the non-zero components, in x, y, z order (q is a
+// constant where this is inlined, so no product and no zero term remains: the
+// compiler has to keep 0 * v, which is not 0 for every v). Used where the
+// terms are not products themselves: there a dropped zero term would let the
+// compiler fuse a product into the sum and change its rounding.
+template <class T>
+__host__ __device__ __forceinline__ T dot_c(int q, T x, T y, T z) {
+    T s = T(0);
+    bool any = false;
+    const int c[3] = {q_cx(q), q_cy(q), q_cz(q)};
+    const T v[3] = {x, y, z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (c[a] == 0) continue;
+        s = any ? (c[a] > 0 ? s + v[a] : s - v[a]) : (c[a] > 0 ? v[a] : -v[a]);
+        any = true;
+    }
+    return s;
+}
+// s += k v for a lattice constant k of -1, 0 or 1
+template <class T>
+__host__ __device__ __forceinline__ void add_k(T& s, int k, T v) {
+    if (k > 0) s += v;
+    else if (k < 0) s -= v;
+}
+
 // 1-D central -> population map along one axis (see back_line in collide27.cuh).
 template <class T>
 struct Line {
@@ -247,9 +273,9 @@ __host__ __device__ void collide_fwd(const T (&f)[27], const CollideParams& P, T
 #pragma unroll
     for (int q = 0; q < 27; ++q) {
         m0 += fo[q];
-        m1x += T(q_cx(q)) * fo[q];
-        m1y += T(q_cy(q)) * fo[q];
-        m1z += T(q_cz(q)) * fo[q];
+        add_k(m1x, q_cx(q), fo[q]);
+        add_k(m1y, q_cy(q), fo[q]);
+        add_k(m1z, q_cz(q), fo[q]);
     }
     const T drho = s.rs - m0;
     const T djx = T(3) * (s.rs * ux - m1x), djy = T(3) * (s.rs * uy - m1y), djz = T(3) * (s.rs * uz - m1z);
@@ -310,7 +336,7 @@ __host__ __device__ void collide_vjp(const CollideTape<T>& s, const CollideParam
     T lfb[27];
 #pragma unroll
     for (int q = 0; q < 27; ++q)
-        lfb[q] = lam_out[q] - ldrho - T(3) * (T(q_cx(q)) * ldj[0] + T(q_cy(q)) * ldj[1] + T(q_cz(q)) * ldj[2]);
+        lfb[q] = lam_out[q] - ldrho - (q == kRest27 ? T(0) : T(3) * dot_c(q, ldj[0], ldj[1], ldj[2]));
 
     // back transform (recompute the x and y passes, then reverse z, y, x)
     T g[3][9], h[27], fb[27];
@@ -471,9 +497,18 @@ __host__ __device__ void collide_vjp(const CollideTape<T>& s, const CollideParam
     const T lr000 = lrho;
 #pragma unroll
     for (int q = 0; q < 27; ++q) {
-        const T cx = T(q_cx(q)), cy = T(q_cy(q)), cz = T(q_cz(q));
-        lam_in[q] = lr000 + cx * lr100 + cy * lr010 + cz * lr001 + cx * cx * lr200 + cy * cy * lr020 + cz * cz * lr002 +
-                    cx * cy * lr110 + cx * cz * lr101 + cy * cz * lr011;
+        const int cx = q_cx(q), cy = q_cy(q), cz = q_cz(q);
+        T l = lr000;
+        add_k(l, cx, lr100);
+        add_k(l, cy, lr010);
+        add_k(l, cz, lr001);
+        add_k(l, cx * cx, lr200);
+        add_k(l, cy * cy, lr020);
+        add_k(l, cz * cz, lr002);
+        add_k(l, cx * cy, lr110);
+        add_k(l, cx * cz, lr101);
+        add_k(l, cy * cz, lr011);
+        lam_in[q] = l;
     }
     lam_F[0] = lF[0];
     lam_F[1] = lF[1];
