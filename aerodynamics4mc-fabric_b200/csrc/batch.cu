@@ -138,7 +138,7 @@ __device__ __forceinline__ void batch_pair(const BrickDesc& b, int cell0) {
 #pragma unroll
         for (int q = 0; q < 27; ++q) {
             const int off = out_offset(G, q, kParity);
-            PairIO<S>::store(base0 + off, base0 + off + 1, st0, st1, q, fl[q], b.sc);
+            PairIO<S>::store(base0 + off, base0 + off + 1, st0, st1, q, fl[q], b.sc, out_scale<false>(q));
         }
         return;
     }
@@ -149,7 +149,7 @@ __device__ __forceinline__ void batch_pair(const BrickDesc& b, int cell0) {
         int c0, d0, c1, d1;
         outgoing_slot(o0, own0, q, kParity, c0, d0);
         outgoing_slot(o1, own0 + 1, q, kParity, c1, d1);
-        PairIO<S>::store(f + (d0 * G.pcells + c0), f + (d1 * G.pcells + c1), st0, st1, q, fl[q], b.sc);
+        PairIO<S>::store(f + (d0 * G.pcells + c0), f + (d1 * G.pcells + c1), st0, st1, q, fl[q], b.sc, out_scale<false>(q));
     }
 }
 

@@ -43,26 +43,26 @@ __device__ __forceinline__ void raw_moments27_x2(const F2 (&f)[27], F2& r000, F2
 #pragma unroll
     for (int l = 0; l < 9; ++l) {
         const F2 fm = f[3 * l + 0], f0 = f[3 * l + 1], fp = f[3 * l + 2];
-        a0[l] = (fm + fp) + f0;
+        a2[l] = fm + fp;
+        a0[l] = a2[l] + f0;
         a1[l] = fp - fm;
-        a2[l] = fp + fm;
     }
     F2 b00[3], b01[3], b02[3], b10[3], b11[3], b20[3];
 #pragma unroll
     for (int ix = 0; ix < 3; ++ix) {
         const int l = 3 * ix;
-        b00[ix] = (a0[l] + a0[l + 2]) + a0[l + 1];
+        b02[ix] = a0[l] + a0[l + 2];
+        b00[ix] = b02[ix] + a0[l + 1];
         b01[ix] = a0[l + 2] - a0[l];
         b10[ix] = (a1[l] + a1[l + 2]) + a1[l + 1];
-        b02[ix] = a0[l + 2] + a0[l];
         b11[ix] = a1[l + 2] - a1[l];
         b20[ix] = (a2[l] + a2[l + 2]) + a2[l + 1];
     }
-    r000 = (b00[0] + b00[2]) + b00[1];
+    r200 = b00[0] + b00[2];
+    r000 = r200 + b00[1];
     r100 = b00[2] - b00[0];
     r010 = (b01[0] + b01[2]) + b01[1];
     r001 = (b10[0] + b10[2]) + b10[1];
-    r200 = b00[2] + b00[0];
     r110 = b01[2] - b01[0];
     r020 = (b02[0] + b02[2]) + b02[1];
     r101 = b10[2] - b10[0];
@@ -70,50 +70,63 @@ __device__ __forceinline__ void raw_moments27_x2(const F2 (&f)[27], F2& r000, F2
     r002 = (b20[0] + b20[2]) + b20[1];
 }
 
-// Orders 0 and 1 only.
+// Post-collision populations are carried as 2^k(q) f_q, k(q) the number of
+// non-zero components of c_q: the halves of the central -> population map
+// (one pair per line and pass, 54 packed products per cell pair) become exact
+// powers of two that the store's own product takes in (16-bit storage) or one
+// product per population (FP32). Scaling by a power of two commutes with
+// every rounding, so the results keep their bits.
+__host__ __device__ constexpr int pop_scale(int q) {
+    return (q_cx(q) != 0 ? 2 : 1) * (q_cy(q) != 0 ? 2 : 1) * (q_cz(q) != 0 ? 2 : 1);
+}
+
+// Orders 0 and 1 of the scaled populations; the first moments come doubled.
 __device__ __forceinline__ void moments01_x2(const F2 (&f)[27], F2& r000, F2& r100, F2& r010, F2& r001) {
+    const F2 half = f2(0.5f);
     F2 a0[9], a1[9];
 #pragma unroll
     for (int l = 0; l < 9; ++l) {
-        a0[l] = (f[3 * l] + f[3 * l + 2]) + f[3 * l + 1];
+        a0[l] = fma2(half, f[3 * l] + f[3 * l + 2], f[3 * l + 1]);
         a1[l] = f[3 * l + 2] - f[3 * l];
     }
     F2 b00[3], b01[3], b10[3];
 #pragma unroll
     for (int ix = 0; ix < 3; ++ix) {
         const int l = 3 * ix;
-        b00[ix] = (a0[l] + a0[l + 2]) + a0[l + 1];
+        b00[ix] = fma2(half, a0[l] + a0[l + 2], a0[l + 1]);
         b01[ix] = a0[l + 2] - a0[l];
-        b10[ix] = (a1[l] + a1[l + 2]) + a1[l + 1];
+        b10[ix] = fma2(half, a1[l] + a1[l + 2], a1[l + 1]);
     }
-    r000 = (b00[0] + b00[2]) + b00[1];
+    r000 = fma2(half, b00[0] + b00[2], b00[1]);
     r100 = b00[2] - b00[0];
-    r010 = (b01[0] + b01[2]) + b01[1];
-    r001 = (b10[0] + b10[2]) + b10[1];
+    r010 = fma2(half, b01[0] + b01[2], b01[1]);
+    r001 = fma2(half, b10[0] + b10[2], b10[1]);
 }
 
-// back_line / back_line_even / back_line_odd of collide27.cuh, packed.
+// back_line / back_line_even / back_line_odd of collide27.cuh, packed; fm and
+// fp come doubled.
 __device__ __forceinline__ void back_line_x2(F2 m0, F2 m1, F2 m2, F2 u, F2& fm, F2& f0, F2& fp) {
     const F2 r1 = fma2(u, m0, m1);
     const F2 r2 = fma2(u, r1 + m1, m2);
-    fm = f2(0.5f) * (r2 - r1);
+    fm = r2 - r1;
     f0 = m0 - r2;
-    fp = f2(0.5f) * (r1 + r2);
+    fp = r1 + r2;
 }
 __device__ __forceinline__ void back_line_even_x2(F2 m0, F2 m2, F2 u, F2& fm, F2& f0, F2& fp) {
     const F2 r1 = u * m0;
     const F2 r2 = fma2(u, r1, m2);
-    fm = f2(0.5f) * (r2 - r1);
+    fm = r2 - r1;
     f0 = m0 - r2;
-    fp = f2(0.5f) * (r1 + r2);
+    fp = r1 + r2;
 }
 __device__ __forceinline__ void back_line_odd_x2(F2 m1, F2 u, F2& fm, F2& f0, F2& fp) {
-    fm = (u - f2(0.5f)) * m1;
+    fm = fma2(f2(2.0f), u, f2(-1.0f)) * m1;
     f0 = (f2(-2.0f) * u) * m1;
-    fp = (u + f2(0.5f)) * m1;
+    fp = fma2(f2(2.0f), u, f2(1.0f)) * m1;
 }
 
-// Collide two fluid cells (lanes x and y of every F2) in place. temp: the
+// Collide two fluid cells (lanes x and y of every F2) in place: the result is
+// pop_scale(q) times the population. temp: the
 // cells' temperatures (read when buoyancy is on); cf*: extra force densities.
 // ok[k] = false: lane k's input was not finite; its populations are then
 // meaningless and the caller reseeds that cell. u: the velocity the
@@ -225,7 +238,8 @@ __device__ __forceinline__ void collide27_x2(F2 (&f)[27], const CollideParams& P
     moments01_x2(f, m0, m1x, m1y, m1z);
     const F2 drho = rs - m0;
     const F2 three = f2(3.0f);
-    const F2 djx = three * (rs * ux - m1x), djy = three * (rs * uy - m1y), djz = three * (rs * uz - m1z);
+    const F2 mh = f2(-0.5f);
+    const F2 djx = three * fma2(m1x, mh, rs * ux), djy = three * fma2(m1y, mh, rs * uy), djz = three * fma2(m1z, mh, rs * uz);
 
     // Guo source pref * w * (3 (c.F - u.F) + 9 (c.u)(c.F)); lanes without force get pref 0
     const bool forced0 = (fx.v.x != 0.0f) | (fy.v.x != 0.0f) | (fz.v.x != 0.0f);
@@ -259,7 +273,7 @@ __device__ __forceinline__ void collide27_x2(F2 (&f)[27], const CollideParams& P
             cu = uz; cf = fz; B = vz;
         }
         const F2 A = fma2(p9 * cu, cf, D);
-        const F2 wq = f2(q_w(q));
+        const F2 wq = f2(q_w(q) * (float)pop_scale(q));
         f[q] = fma2(wq, A + B, f[q]);
         f[26 - q] = fma2(wq, A - B, f[26 - q]);
     }

@@ -349,11 +349,11 @@ __global__ void __launch_bounds__(kIpaWarps * 32, AERO_IPA_MIN_BLOCKS)
                 int c, d;
                 if (pass0) {
                     incoming_slot(o0, own0, q, kParity, (w0 >> q) & 1u, c, d);
-                    fl[q].v.x = S::load(f + (d * G.pcells + c), q, a.sc);
+                    fl[q].v.x = S::load(f + (d * G.pcells + c), q, a.sc) * (float)pop_scale(q);
                 }
                 if (pass1) {
                     incoming_slot(o1, own1, q, kParity, (w1 >> q) & 1u, c, d);
-                    fl[q].v.y = S::load(f + (d * G.pcells + c), q, a.sc);
+                    fl[q].v.y = S::load(f + (d * G.pcells + c), q, a.sc) * (float)pop_scale(q);
                 }
             }
         }
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(kIpaWarps * 32, AERO_IPA_MIN_BLOCKS)
 #pragma unroll
             for (int q = 0; q < 27; ++q) {
                 const int off = out_offset(G, q, kParity);
-                PairIO<S>::store(base0 + off, base0 + off + 1, st0, st1, q, fl[q], a.sc);
+                PairIO<S>::store(base0 + off, base0 + off + 1, st0, st1, q, fl[q], a.sc, out_scale<false>(q));
             }
         } else {
             const NeighbourOffsets o0 = neighbour_offsets(G, x, y, z0);
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(kIpaWarps * 32, AERO_IPA_MIN_BLOCKS)
                 int c0, d0, c1, d1;
                 outgoing_slot(o0, own0, q, kParity, c0, d0);
                 outgoing_slot(o1, own1, q, kParity, c1, d1);
-                PairIO<S>::store(f + (d0 * G.pcells + c0), f + (d1 * G.pcells + c1), st0, st1, q, fl[q], a.sc);
+                PairIO<S>::store(f + (d0 * G.pcells + c0), f + (d1 * G.pcells + c1), st0, st1, q, fl[q], a.sc, out_scale<false>(q));
             }
         }
     }

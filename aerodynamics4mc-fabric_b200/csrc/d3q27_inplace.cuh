@@ -148,6 +148,41 @@ __device__ __forceinline__ void reseed_push(typename S::T* f, const IpArgs& a, l
                       z, a.g.nx, a.g.ny, a.g.nz, wrap_mask, parity, a.cur.u_last);
 }
 
+// A cell that was fluid at streaming and is solid now: its streamed
+// populations go out uncollided. A pair's two outgoing slots are its two
+// incoming ones swapped (a bounced pull reads a slot this cell does not write),
+// so each pair is read before it is written. Out of line: rare.
+template <class S>
+static __device__ __noinline__ void pass_through_ip(typename S::T* __restrict__ f, uint32_t w, float fp16_scale, int x, int y,
+                                                     int z, int nx, int ny, int nz, int wrap_mask, int parity) {
+    const PadGeom g = make_pad_geom(nx, ny, nz, wrap_mask);
+    const NeighbourOffsets o = neighbour_offsets(g, x, y, z);
+    const int own = pad_index(g, x, y, z);
+    const Fp16Scale sc{fp16_scale, 1.0f / fp16_scale};
+#pragma unroll 1
+    for (int q = 14; q < 27; ++q) {
+        float v[2];
+        for (int k = 0; k < 2; ++k) {
+            const int p = k ? 26 - q : q;
+            int c, d;
+            incoming_slot(o, own, p, parity, (w >> p) & 1u, c, d);
+            v[k] = S::load(f + (long long)d * g.pcells + c, p, sc);
+        }
+        for (int k = 0; k < 2; ++k) {
+            const int p = k ? 26 - q : q;
+            int c, d;
+            outgoing_slot(o, own, p, parity, c, d);
+            S::store(f + (long long)d * g.pcells + c, p, v[k], sc);
+        }
+    }
+}
+
+template <class S>
+__device__ __forceinline__ void pass_through(typename S::T* f, const IpArgs& a, uint32_t w, int x, int y, int z, int parity) {
+    const int wrap_mask = a.g.wrap[0] | (a.g.wrap[1] << 1) | (a.g.wrap[2] << 2);
+    pass_through_ip<S>(f, w, a.sc.scale, x, y, z, a.g.nx, a.g.ny, a.g.nz, wrap_mask, parity);
+}
+
 // Velocities a two-cell step leaves for the temperature transport: the
 // collision's on collided lanes, 0 on lanes that are solid now or were at
 // the streaming call (a reseeded lane records its own in reseed_push; a
@@ -237,7 +272,8 @@ __global__ void __launch_bounds__(128) step_ip_kernel(typename S::T* __restrict_
 
 // Loads and stores of two cells' populations of one direction: at two
 // addresses, or (load2 / store2) as one aligned 2-element vector at p (the
-// first cell's slot; the second cell's is the next element).
+// first cell's slot; the second cell's is the next element). A store takes
+// `by` times the value, an exact power of two (out_scale).
 template <class S>
 struct PairIO;
 template <>
@@ -253,12 +289,14 @@ struct PairIO<StoreF32> {
         if (fix) r.y = __ldg(p1);
         return F2{r};
     }
-    __device__ __forceinline__ static void store(float* p0, float* p1, bool s0, bool s1, int, F2 v, const Fp16Scale&) {
+    __device__ __forceinline__ static F2 unscaled(F2 v, float by) { return by == 1.0f ? v : f2(by) * v; }
+    __device__ __forceinline__ static void store(float* p0, float* p1, bool s0, bool s1, int, F2 v, const Fp16Scale&, float by = 1.0f) {
+        v = unscaled(v, by);
         if (s0) *p0 = v.v.x;
         if (s1) *p1 = v.v.y;
     }
-    __device__ __forceinline__ static void store2(float* p, int, F2 v, const Fp16Scale&) {
-        *reinterpret_cast<float2*>(p) = v.v;
+    __device__ __forceinline__ static void store2(float* p, int, F2 v, const Fp16Scale&, float by = 1.0f) {
+        *reinterpret_cast<float2*>(p) = unscaled(v, by).v;
     }
 };
 template <>
@@ -267,8 +305,8 @@ struct PairIO<StoreF16Dev> {
         const float w = q_w(q), k = w * s.inv_scale;
         return F2{__ffma2_rn(h, make_float2(k, k), make_float2(w, w))};
     }
-    __device__ __forceinline__ static float2 encode(F2 v, int q, const Fp16Scale& s) {
-        const float k = s.scale * (1.0f / q_w(q));
+    __device__ __forceinline__ static float2 encode(F2 v, int q, const Fp16Scale& s, float by) {
+        const float k = s.scale * (1.0f / q_w(q)) * by;
         return __ffma2_rn(v.v, make_float2(k, k), make_float2(-s.scale, -s.scale));
     }
     __device__ __forceinline__ static F2 load(const __half* p0, const __half* p1, int q, const Fp16Scale& s) {
@@ -283,13 +321,13 @@ struct PairIO<StoreF16Dev> {
         if (fix) y = __ldg(p1);
         return decode(make_float2(__low2float(r), __half2float(y)), q, s);
     }
-    __device__ __forceinline__ static void store(__half* p0, __half* p1, bool s0, bool s1, int q, F2 v, const Fp16Scale& s) {
-        const float2 h = encode(v, q, s);
+    __device__ __forceinline__ static void store(__half* p0, __half* p1, bool s0, bool s1, int q, F2 v, const Fp16Scale& s, float by = 1.0f) {
+        const float2 h = encode(v, q, s, by);
         if (s0) *p0 = __float2half_rn(h.x);
         if (s1) *p1 = __float2half_rn(h.y);
     }
-    __device__ __forceinline__ static void store2(__half* p, int q, F2 v, const Fp16Scale& s) {
-        const float2 h = encode(v, q, s);
+    __device__ __forceinline__ static void store2(__half* p, int q, F2 v, const Fp16Scale& s, float by = 1.0f) {
+        const float2 h = encode(v, q, s, by);
         *reinterpret_cast<__half2*>(p) = __floats2half2_rn(h.x, h.y);
     }
 };
@@ -300,8 +338,8 @@ struct PairIO<StoreI16Dev> {
         const float w = q_w(q), k = w * s.inv_scale;
         return F2{__ffma2_rn(h, make_float2(k, k), make_float2(w, w))};
     }
-    __device__ __forceinline__ static float2 encode(F2 v, int q, const Fp16Scale& s) {
-        const float k = s.scale * (1.0f / q_w(q));
+    __device__ __forceinline__ static float2 encode(F2 v, int q, const Fp16Scale& s, float by) {
+        const float k = s.scale * (1.0f / q_w(q)) * by;
         return __ffma2_rn(v.v, make_float2(k, k), make_float2(-s.scale, -s.scale));
     }
     __device__ __forceinline__ static F2 load(const short* p0, const short* p1, int q, const Fp16Scale& s) {
@@ -316,13 +354,13 @@ struct PairIO<StoreI16Dev> {
         if (fix) r = (r & 0xFFFFu) | ((unsigned)(unsigned short)__ldg(p1) << 16);
         return decode(s16x2_to_float2(r), q, s);
     }
-    __device__ __forceinline__ static void store(short* p0, short* p1, bool s0, bool s1, int q, F2 v, const Fp16Scale& s) {
-        const float2 h = encode(v, q, s);
+    __device__ __forceinline__ static void store(short* p0, short* p1, bool s0, bool s1, int q, F2 v, const Fp16Scale& s, float by = 1.0f) {
+        const float2 h = encode(v, q, s, by);
         if (s0) *p0 = sat_round_s16(h.x);
         if (s1) *p1 = sat_round_s16(h.y);
     }
-    __device__ __forceinline__ static void store2(short* p, int q, F2 v, const Fp16Scale& s) {
-        const float2 h = encode(v, q, s);
+    __device__ __forceinline__ static void store2(short* p, int q, F2 v, const Fp16Scale& s, float by = 1.0f) {
+        const float2 h = encode(v, q, s, by);
         *reinterpret_cast<short2*>(p) = make_short2(sat_round_s16(h.x), sat_round_s16(h.y));
     }
 };
@@ -359,23 +397,35 @@ __host__ __device__ constexpr bool out_pair_aligned(int q) {
 // (one of two per direction, by the bounce-back bit; the second cell's slots
 // one element after the first's).
 // A cell that is fluid at the streaming call and solid now is not collided:
-// its streamed populations pass through (reloaded from its incoming slots,
-// which only this cell writes, before any store). A lane whose input is not
-// finite is reseeded.
+// its streamed populations pass through (read again from its incoming slots,
+// which only this cell writes). A lane whose input is not finite is reseeded.
+// Both happen after the other lanes' stores.
 #ifndef AERO_IP2_MIN_BLOCKS
 #define AERO_IP2_MIN_BLOCKS 5
 #endif
 #ifndef AERO_IP2X_MIN_BLOCKS
 #define AERO_IP2X_MIN_BLOCKS 4
 #endif
+// Place of a two-cell thread (volatile: evaluated where it is called).
+__device__ __forceinline__ void pair_coords(int& x, int& y, int& z0) {
+    int t, b, n;
+    asm volatile("mov.u32 %0, %%tid.x;\n\tmov.u32 %1, %%ctaid.x;\n\tmov.u32 %2, %%ntid.x;" : "=r"(t), "=r"(b), "=r"(n));
+    asm volatile("mov.u32 %0, %%ctaid.y;\n\tmov.u32 %1, %%ctaid.z;" : "=r"(y), "=r"(x));
+    z0 = 2 * (b * n + t);
+}
+
+// Factor from a collision's result to the population it stores.
+template <bool kExact>
+__host__ __device__ constexpr float out_scale(int q) { return kExact ? 1.0f : 1.0f / (float)pop_scale(q); }
+
 template <class S, bool kExact, int kParity, bool kTransport>
 __global__ void __launch_bounds__(128, kExact ? AERO_IP2X_MIN_BLOCKS : AERO_IP2_MIN_BLOCKS) step_ip2_kernel(typename S::T* __restrict__ f, IpArgs a) {
     // launched after the transport (and the face pre-fill) with launch_pdl
     pdl_trigger();
     pdl_wait();
     const PadGeom& G = a.g;
-    const int z0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
-    const int y = blockIdx.y, x = blockIdx.z;
+    int x, y, z0;
+    pair_coords(x, y, z0);
     float tn[2] = {0.0f, 0.0f};
     if (kTransport) {
         const int z_begin = 2 * blockIdx.x * blockDim.x;
@@ -383,7 +433,7 @@ __global__ void __launch_bounds__(128, kExact ? AERO_IP2X_MIN_BLOCKS : AERO_IP2_
         fused_transport<2>(a, x, y, z_begin, min(2 * (int)blockDim.x, G.nz - z_begin), zs, tn);
     }
     if (z0 >= G.nz) return;
-    const long long cell0 = ((long long)x * G.ny + y) * G.nz + z0;
+    long long cell0 = ((long long)x * G.ny + y) * G.nz + z0;
     const bool has1 = z0 + 1 < G.nz;
     const uint32_t w0 = a.flags_prev[cell0];
     const uint32_t w1 = has1 ? a.flags_prev[cell0 + 1] : kFlagSelfSolid;
@@ -397,8 +447,8 @@ __global__ void __launch_bounds__(128, kExact ? AERO_IP2X_MIN_BLOCKS : AERO_IP2_
     }
     const bool pass0 = live0 && a.obstacle_cur[cell0] != 0;
     const bool pass1 = live1 && a.obstacle_cur[cell0 + 1] != 0;
-    const int own0 = pad_index(G, x, y, z0);
-    const int own1 = own0 + 1;  // z0 + 1 (the ghost cell when z0 + 1 == nz: inside the padded array)
+    int own0 = pad_index(G, x, y, z0);
+    int own1 = own0 + 1;  // z0 + 1 (the ghost cell when z0 + 1 == nz: inside the padded array)
     const bool flat = no_wrap(G, x, y, z0) && (!has1 || no_wrap(G, x, y, z0 + 1));
     typename S::T* __restrict__ base0 = f + own0;
     F2 fl[27];
@@ -441,52 +491,51 @@ __global__ void __launch_bounds__(128, kExact ? AERO_IP2X_MIN_BLOCKS : AERO_IP2_
     F2 uc[3];
     if (kExact) exact::collide27_exact_x2(fl, a.cp, t, cfx, cfy, cfz, ok, uc);
     else collide27_x2(fl, a.cp, t, cfx, cfy, cfz, ok, uc);
+    // the pair's place again from the launch registers: kept through the
+    // collision it would be spilled
+    pair_coords(x, y, z0);
+    cell0 = ((long long)x * G.ny + y) * G.nz + z0;
+    own0 = pad_index(G, x, y, z0);
+    own1 = own0 + 1;
+    base0 = f + own0;
     record_u2(a.cur, cell0, has1, live0 && !pass0 && ok[0], live1 && !pass1 && ok[1], live0 && !ok[0] && !pass0,
               live1 && !ok[1] && !pass1, uc);
-    if (pass0 || pass1) {
-        const NeighbourOffsets o0 = neighbour_offsets(G, x, y, z0);
-        const NeighbourOffsets o1 = neighbour_offsets(G, x, y, has1 ? z0 + 1 : z0);
-#pragma unroll
-        for (int q = 0; q < 27; ++q) {
-            int c, d;
-            if (pass0) {
-                incoming_slot(o0, own0, q, kParity, (w0 >> q) & 1u, c, d);
-                fl[q].v.x = S::load(f + (d * G.pcells + c), q, a.sc);
-            }
-            if (pass1) {
-                incoming_slot(o1, own1, q, kParity, (w1 >> q) & 1u, c, d);
-                fl[q].v.y = S::load(f + (d * G.pcells + c), q, a.sc);
-            }
-        }
-    }
-    const bool st0 = live0 && (ok[0] || pass0), st1 = live1 && (ok[1] || pass1);
-    if (live0 && !ok[0] && !pass0) reseed_push<S>(f, a, cell0, x, y, z0, kParity);
-    if (live1 && !ok[1] && !pass1) reseed_push<S>(f, a, cell0 + 1, x, y, z0 + 1, kParity);
+    const bool st0 = live0 && ok[0] && !pass0, st1 = live1 && ok[1] && !pass1;
     if (flat) {
         if (st0 && st1) {
 #pragma unroll
             for (int q = 0; q < 27; ++q) {
                 const int off = a.off_out[q];
-                if (out_pair_aligned(q)) PairIO<S>::store2(base0 + off, q, fl[q], a.sc);
-                else PairIO<S>::store(base0 + off, base0 + off + 1, true, true, q, fl[q], a.sc);
+                if (out_pair_aligned(q)) PairIO<S>::store2(base0 + off, q, fl[q], a.sc, out_scale<kExact>(q));
+                else PairIO<S>::store(base0 + off, base0 + off + 1, true, true, q, fl[q], a.sc, out_scale<kExact>(q));
             }
         } else {
 #pragma unroll
             for (int q = 0; q < 27; ++q) {
                 const int off = a.off_out[q];
-                PairIO<S>::store(base0 + off, base0 + off + 1, st0, st1, q, fl[q], a.sc);
+                PairIO<S>::store(base0 + off, base0 + off + 1, st0, st1, q, fl[q], a.sc, out_scale<kExact>(q));
             }
         }
-        return;
-    }
-    const NeighbourOffsets o0 = neighbour_offsets(G, x, y, z0);
-    const NeighbourOffsets o1 = neighbour_offsets(G, x, y, has1 ? z0 + 1 : z0);
+    } else {
+        const NeighbourOffsets o0 = neighbour_offsets(G, x, y, z0);
+        const NeighbourOffsets o1 = neighbour_offsets(G, x, y, has1 ? z0 + 1 : z0);
 #pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        int c0, d0, c1, d1;
-        outgoing_slot(o0, own0, q, kParity, c0, d0);
-        outgoing_slot(o1, own1, q, kParity, c1, d1);
-        PairIO<S>::store(f + (d0 * G.pcells + c0), f + (d1 * G.pcells + c1), st0, st1, q, fl[q], a.sc);
+        for (int q = 0; q < 27; ++q) {
+            int c0, d0, c1, d1;
+            outgoing_slot(o0, own0, q, kParity, c0, d0);
+            outgoing_slot(o1, own1, q, kParity, c1, d1);
+            PairIO<S>::store(f + (d0 * G.pcells + c0), f + (d1 * G.pcells + c1), st0, st1, q, fl[q], a.sc, out_scale<kExact>(q));
+        }
+    }
+    // the rare lanes last, when no population is held any more (every slot
+    // they read or write is their own)
+    if (live0 && !st0) {
+        if (pass0) pass_through<S>(f, a, a.flags_prev[cell0], x, y, z0, kParity);
+        else reseed_push<S>(f, a, cell0, x, y, z0, kParity);
+    }
+    if (live1 && !st1) {
+        if (pass1) pass_through<S>(f, a, a.flags_prev[cell0 + 1], x, y, z0 + 1, kParity);
+        else reseed_push<S>(f, a, cell0 + 1, x, y, z0 + 1, kParity);
     }
 }
 
