@@ -15,7 +15,7 @@
 //     is the identity, so the sums are unchanged;
 //   * only the moments the collision reads are formed (the reference computes
 //     all 27 pre-collision central moments but uses the second-order six).
-// Flops per cell are about a third of the reference's dense loops; the
+// The operations left are about a quarter of the reference dense loops; the
 // collision is still ALU-heavier than the factorised form (collide27.cuh).
 #pragma once
 
@@ -29,25 +29,7 @@ __device__ __forceinline__ float rmax(float a, float b) { return (a < b) ? b : a
 __device__ __forceinline__ float rmin(float a, float b) { return (b < a) ? b : a; }
 __device__ __forceinline__ float rclamp(float v, float lo, float hi) { return rmin(hi, rmax(lo, v)); }
 
-__host__ __device__ constexpr int cval(int i) { return i - 1; }
 __host__ __device__ constexpr int binom2(int n, int k) { return (k < 0 || k > n) ? 0 : ((n <= 1 || k == 0 || k == n) ? 1 : 2); }
-
-// c.u for direction q, summed x, y, z skipping zero components.
-__device__ __forceinline__ float cdot(int q, float ux, float uy, float uz) {
-    const int cx = q_cx(q), cy = q_cy(q), cz = q_cz(q);
-    float s = 0.0f;
-    bool any = false;
-    if (cx != 0) { s = cx > 0 ? ux : -ux; any = true; }
-    if (cy != 0) { const float t = cy > 0 ? uy : -uy; s = any ? s + t : t; any = true; }
-    if (cz != 0) { const float t = cz > 0 ? uz : -uz; s = any ? s + t : t; any = true; }
-    return s;
-}
-
-// feq(q, rho, u) = w rho (1 + cu + 0.5 cu^2 - 1.5 u.u), cu = 3 c.u
-__device__ __forceinline__ float feq(int q, float rho, float ux, float uy, float uz, float uu) {
-    const float cu = 3.0f * cdot(q, ux, uy, uz);
-    return q_w(q) * rho * (1.0f + cu + 0.5f * cu * cu - 1.5f * uu);
-}
 
 // Signed sum over q (in q order) of f[q] * cx^a cy^b cz^c, terms with a zero
 // coefficient skipped: the reference's raw moment / momentum sums.
@@ -67,9 +49,195 @@ __device__ __forceinline__ float qsum(const float (&f)[27]) {
     return s;
 }
 
-struct ExactOut {
-    float rho, ux, uy, uz;
+// ---- the part after the cumulant relaxation, over one cell (V = float) or
+// two (V = X2 of collide27_exact_x2.cuh). It performs the reference's roundings
+// and drops what rounds nothing:
+//   * opposite directions share their products: c.u and c.F only change sign,
+//     and every rounding commutes with a change of sign;
+//   * the products of velocity powers are formed once, without the binomial
+//     coefficient (1, 2, 4, 8), which goes into the sum's fused multiply-add
+//     (an exact product);
+//   * the 1-D inverse rows {0,-1/2,1/2}, {1,0,-1}, {0,1/2,1/2} run as plain
+//     sums: populations are carried as 2^k(q) f_q (k(q): non-zero components
+//     of c_q; those with c_x = -1 negated as well, so that c_x = -1 and +1
+//     share the sum over R[1]) until a fused multiply-add takes them up.
+// The 128^3 step (FP32 in-place, two cells per thread, B200) went from 204.8 to
+// 188.7 us, its stream-collide launch from 174.9 to 160.3, without spills.
+struct PlainMul {
+    __device__ __forceinline__ float operator()(float a, float b) const { return a * b; }
 };
+template <class V>
+__device__ __forceinline__ V splat(float a);
+template <>
+__device__ __forceinline__ float splat<float>(float a) { return a; }
+// c * x + s for a power of two c: the reference's product and sum
+__device__ __forceinline__ float fma_pow2(float c, float x, float s) { return fmaf(c, x, s); }
+__device__ __forceinline__ float mul_pow2(float c, float x) { return c * x; }
+
+// 2^k(q), and the sign the carried population has
+__host__ __device__ constexpr float carried(int q) {
+    return (q_cx(q) < 0 ? -1.0f : 1.0f) * (q_cx(q) != 0 ? 2.0f : 1.0f) * (q_cy(q) != 0 ? 2.0f : 1.0f) * (q_cz(q) != 0 ? 2.0f : 1.0f);
+}
+
+// c_q . (x, y, z) for q > 13 (the first non-zero component is +1)
+template <class V>
+__device__ __forceinline__ V cdot_pos(int q, V x, V y, V z) {
+    const int cx = q_cx(q), cy = q_cy(q), cz = q_cz(q);
+    V s = cx ? x : (cy ? y : z);
+    if (cx && cy) s = cy > 0 ? s + y : s - y;
+    if ((cx || cy) && cz) s = cz > 0 ? s + z : s - z;
+    return s;
+}
+
+// Signed sum over q (in q order) of the carried populations' true values
+// times c_A (A: 0 none, 1 x, 2 y, 3 z).
+template <int A, class V>
+__device__ __forceinline__ V carried_sum(const V (&fc)[27]) {
+    V s;
+    bool first = true;
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        const int c = A == 0 ? 1 : (A == 1 ? q_cx(q) : (A == 2 ? q_cy(q) : q_cz(q)));
+        if (c == 0) continue;
+        const float k = (float)c / carried(q);
+        s = first ? mul_pow2(k, fc[q]) : fma_pow2(k, fc[q], s);
+        first = false;
+    }
+    return s;
+}
+
+// Carried populations fc from the post-collision central moments K
+// (central_to_raw, raw_to_populations).
+template <class V, class M>
+__device__ __forceinline__ void central_to_populations(const M& mul, const V (&K)[3][3][3], V ux, V uy, V uz, V (&fc)[27]) {
+    const V px[3] = {ux, ux, mul(ux, ux)}, py[3] = {uy, uy, mul(uy, uy)}, pz[3] = {uz, uz, mul(uz, uz)};
+    // entry R[a][b][c] = sum over (p, q, r) <= (a, b, c), p + q + r even, of
+    // binomials * ((ux^(a-p) uy^(b-q)) uz^(c-r)) * K[p][q][r]
+    V R[3][3][3];
+    auto raw = [&](int a, int b, int c) {
+        V sum;
+        bool first = true;
+#pragma unroll
+        for (int p = 0; p <= a; ++p)
+#pragma unroll
+            for (int qq = 0; qq <= b; ++qq)
+#pragma unroll
+                for (int r = 0; r <= c; ++r) {
+                    if (((p + qq + r) & 1) != 0) continue;  // odd-order post-collision moments are zero
+                    const int i = a - p, j = b - qq, k = c - r;
+                    V t = K[p][qq][r];
+                    if (i && j && k) t = mul(mul(mul(px[i], py[j]), pz[k]), t);
+                    else if (i && j) t = mul(mul(px[i], py[j]), t);
+                    else if (i && k) t = mul(mul(px[i], pz[k]), t);
+                    else if (j && k) t = mul(mul(py[j], pz[k]), t);
+                    else if (i) t = mul(px[i], t);
+                    else if (j) t = mul(py[j], t);
+                    else if (k) t = mul(pz[k], t);
+                    const int coef = binom2(a, p) * binom2(b, qq) * binom2(c, r);
+                    sum = first ? t : (coef == 1 ? sum + t : fma_pow2((float)coef, t, sum));
+                    first = false;
+                }
+        R[a][b][c] = sum;
+    };
+    // signs of the two non-zero entries of inverse row i (times 2 for i != 1)
+    constexpr int lo[3] = {1, 0, 1}, s_lo[3] = {-1, 1, 1}, s_hi[3] = {1, -1, 1};
+    // sum + / - the entries of raw slab a for the (iy, iz) population, in (b, c)
+    // order; sign: of the slab
+    auto slab = [&](int a, int iy, int iz, int sign, bool start, V s) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int sg = sign * (b ? s_hi[iy] : s_lo[iy]) * (c ? s_hi[iz] : s_lo[iz]);
+                const V r = R[a][b ? 2 : lo[iy]][c ? 2 : lo[iz]];
+                if (start && b == 0 && c == 0) s = sg > 0 ? r : -r;
+                else s = sg > 0 ? s + r : s - r;
+            }
+        return s;
+    };
+    // c_x = 0 reads only R[0] and R[2], the others only R[1] and R[2]: R[0] and
+    // R[1] are never live together
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            raw(0, b, c);
+            raw(2, b, c);
+        }
+#pragma unroll
+    for (int iy = 0; iy < 3; ++iy)
+#pragma unroll
+        for (int iz = 0; iz < 3; ++iz) fc[9 + iy * 3 + iz] = slab(2, iy, iz, -1, false, slab(0, iy, iz, 1, true, R[0][0][0]));
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) raw(1, b, c);
+#pragma unroll
+    for (int iy = 0; iy < 3; ++iy)
+#pragma unroll
+        for (int iz = 0; iz < 3; ++iz) {
+            const V s = slab(1, iy, iz, 1, true, R[1][0][0]);
+            fc[iy * 3 + iz] = slab(2, iy, iz, -1, false, s);       // negated
+            fc[18 + iy * 3 + iz] = slab(2, iy, iz, 1, false, s);
+        }
+}
+
+// feq(q) / w and feq(26 - q) / w, q > 13: rho (1 + cu + 0.5 cu^2 - 1.5 u.u), cu = 3 c.u
+template <class V, class M>
+__device__ __forceinline__ void feq_pair(const M& mul, int q, V wr, V ux, V uy, V uz, V uu15, V& e, V& eo) {
+    const V cu = mul(splat<V>(3.0f), cdot_pos(q, ux, uy, uz));
+    const V t = mul(mul(splat<V>(0.5f), cu), cu), one = splat<V>(1.0f);
+    e = mul(wr, ((one + cu) + t) - uu15);
+    eo = mul(wr, ((one - cu) + t) - uu15);
+}
+
+// w_q classes by the number of non-zero components: 0, 1, 2, 3
+__host__ __device__ constexpr int w_class(int q) { return (q_cx(q) != 0) + (q_cy(q) != 0) + (q_cz(q) != 0); }
+__host__ __device__ constexpr int w_member(int k) { return k == 0 ? 13 : (k == 1 ? 14 : (k == 2 ? 17 : 26)); }
+
+// fc (carried) -> f: the conservation fix-up.
+template <class V, class M>
+__device__ __forceinline__ void conserve(const M& mul, const V (&fc)[27], V rho, V ux, V uy, V uz, V rho_c, V uxc, V uyc, V uzc,
+                                         V (&f)[27]) {
+    const V uu15 = mul(splat<V>(1.5f), (mul(ux, ux) + mul(uy, uy)) + mul(uz, uz));
+    const V uuc15 = mul(splat<V>(1.5f), (mul(uxc, uxc) + mul(uyc, uyc)) + mul(uzc, uzc));
+    V wr[4], wc[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        wr[k] = mul(splat<V>(q_w(w_member(k))), rho);
+        wc[k] = mul(splat<V>(q_w(w_member(k))), rho_c);
+    }
+    const V one = splat<V>(1.0f);
+    f[13] = fc[13] + (mul(wr[0], one - uu15) - mul(wc[0], one - uuc15));
+#pragma unroll
+    for (int q = 14; q < 27; ++q) {
+        V e, eo, g, go;
+        feq_pair(mul, q, wr[w_class(q)], ux, uy, uz, uu15, e, eo);
+        feq_pair(mul, q, wc[w_class(q)], uxc, uyc, uzc, uuc15, g, go);
+        f[q] = fma_pow2(1.0f / carried(q), fc[q], e - g);
+        f[26 - q] = fma_pow2(1.0f / carried(26 - q), fc[26 - q], eo - go);
+    }
+}
+
+// f += Guo source, pref w ((c.F - u.F) / cs2 + (c.u)(c.F) / cs4)
+template <class V, class M, class Put>
+__device__ __forceinline__ void guo(const M& mul, V pref, V ux, V uy, V uz, V fx, V fy, V fz, const V (&f)[27], Put put) {
+    const float inv_cs2 = 1.0f / kCs2f;
+    const float inv_cs4 = inv_cs2 * inv_cs2;
+    const V uf = (mul(ux, fx) + mul(uy, fy)) + mul(uz, fz);
+    V pw[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) pw[k] = mul(pref, splat<V>(q_w(w_member(k))));
+    put(13, f[13] - mul(pw[0], mul(uf, splat<V>(inv_cs2))));
+#pragma unroll
+    for (int q = 14; q < 27; ++q) {
+        const V cf = cdot_pos(q, fx, fy, fz);
+        const V d = mul(mul(cdot_pos(q, ux, uy, uz), cf), splat<V>(inv_cs4));
+        const V w = pw[w_class(q)];
+        put(q, f[q] + mul(w, mul(cf - uf, splat<V>(inv_cs2)) + d));
+        put(26 - q, f[26 - q] + mul(w, d - mul(cf + uf, splat<V>(inv_cs2))));
+    }
+}
 
 // Collide one fluid cell in place (benchmark-mode reference collide: no fan
 // forcing, no edge nudge, no sponge). Returns false, with f untouched, when
@@ -190,92 +358,15 @@ __device__ __forceinline__ bool collide27_exact(float (&f)[27], const CollidePar
                       2.0f * k011 * k011 * k200 + 8.0f * k110 * k101 * k011) * ir * ir;
     }
 
-    // central_to_raw: R[a][b][c] = sum over non-zero K[p][q][r], (p,q,r) <= (a,b,c),
-    // of ((((binom * ux^(a-p)) * uy^(b-q)) * uz^(c-r)) * K[p][q][r]).
-    const float upx[3] = {1.0f, ux, ux * ux};
-    const float upy[3] = {1.0f, uy, uy * uy};
-    const float upz[3] = {1.0f, uz, uz * uz};
-    float R[3][3][3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                float sum = 0.0f;
-                bool first = true;
-#pragma unroll
-                for (int p = 0; p <= a; ++p)
-#pragma unroll
-                    for (int qq = 0; qq <= b; ++qq)
-#pragma unroll
-                        for (int r = 0; r <= c; ++r) {
-                            if (((p + qq + r) & 1) != 0) continue;  // odd-order post-collision moments are zero
-                            const float coeff = float(binom2(a, p) * binom2(b, qq) * binom2(c, r));
-                            float t = coeff;
-                            if (a - p > 0) t = t * upx[a - p];
-                            if (b - qq > 0) t = t * upy[b - qq];
-                            if (c - r > 0) t = t * upz[c - r];
-                            t = t * K[p][qq][r];
-                            sum = first ? t : sum + t;
-                            first = false;
-                        }
-                R[a][b][c] = sum;
-            }
-
-    // raw_to_populations with the 1-D inverse rows {0,-1/2,1/2}, {1,0,-1}, {0,1/2,1/2}.
-    // The coefficient products are powers of two, so coef*R is exact and the
-    // fused multiply-add rounds exactly like the reference's multiply then add.
-    constexpr float inv1[3][3] = {{0.0f, -0.5f, 0.5f}, {1.0f, 0.0f, -1.0f}, {0.0f, 0.5f, 0.5f}};
+    const PlainMul mul;
     float fc[27];
-#pragma unroll
-    for (int ix = 0; ix < 3; ++ix)
-#pragma unroll
-        for (int iy = 0; iy < 3; ++iy)
-#pragma unroll
-            for (int iz = 0; iz < 3; ++iz) {
-                float sum = 0.0f;
-                bool first = true;
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int b = 0; b < 3; ++b)
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            const float coef = inv1[ix][a] * inv1[iy][b] * inv1[iz][c];
-                            if (coef == 0.0f) continue;
-                            sum = first ? coef * R[a][b][c] : fmaf(coef, R[a][b][c], sum);
-                            first = false;
-                        }
-                fc[(ix * 3 + iy) * 3 + iz] = sum;
-            }
-
-    // Conservation fix-up.
-    const float rho_c = qsum<0, 0, 0>(fc);
-    const float mx_c = qsum<1, 0, 0>(fc);
-    const float my_c = qsum<0, 1, 0>(fc);
-    const float mz_c = qsum<0, 0, 1>(fc);
-    const float rho_cs = rmax(1e-6f, rho_c);
-    const float uxc = mx_c / rho_cs, uyc = my_c / rho_cs, uzc = mz_c / rho_cs;
-    const float uu = ux * ux + uy * uy + uz * uz;
-    const float uuc = uxc * uxc + uyc * uyc + uzc * uzc;
-#pragma unroll
-    for (int q = 0; q < 27; ++q) fc[q] += feq(q, rho_safe, ux, uy, uz, uu) - feq(q, rho_cs, uxc, uyc, uzc, uuc);
-
+    central_to_populations(mul, K, ux, uy, uz, fc);
+    const float rho_cs = rmax(1e-6f, carried_sum<0>(fc));
+    const float uxc = carried_sum<1>(fc) / rho_cs, uyc = carried_sum<2>(fc) / rho_cs, uzc = carried_sum<3>(fc) / rho_cs;
+    conserve(mul, fc, rho_safe, ux, uy, uz, rho_cs, uxc, uyc, uzc, f);
     if (forced) {
-        const float inv_cs2 = 1.0f / kCs2f;
-        const float inv_cs4 = inv_cs2 * inv_cs2;
         const float pref = rmax(0.0f, 1.0f - 0.5f * rclamp(omega_off, 0.0f, 1.999f));
-        const float u_force = ux * fx + uy * fy + uz * fz;
-#pragma unroll
-        for (int q = 0; q < 27; ++q) {
-            const float cu = cdot(q, ux, uy, uz);
-            const float c_force = cdot(q, fx, fy, fz);
-            f[q] = fc[q] + pref * q_w(q) * ((c_force - u_force) * inv_cs2 + cu * c_force * inv_cs4);
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < 27; ++q) f[q] = fc[q];
+        guo(mul, pref, ux, uy, uz, fx, fy, fz, f, [&](int q, float v) { f[q] = v; });
     }
     return true;
 }

@@ -70,9 +70,17 @@ __device__ __forceinline__ X2 rmin2(X2 v, float c) { return x2(rmin(v.v.x, c), r
 __device__ __forceinline__ X2 rclamp2(X2 v, float lo, float hi) { return x2(rclamp(v.v.x, lo, hi), rclamp(v.v.y, lo, hi)); }
 __device__ __forceinline__ X2 div2x(X2 a, X2 b) { return x2(a.v.x / b.v.x, a.v.y / b.v.y); }
 
+template <>
+__device__ __forceinline__ X2 splat<X2>(float a) { return x2(a); }
+__device__ __forceinline__ X2 fma_pow2(float c, X2 x, X2 s) { return xfma(x2(c), x, s); }
+__device__ __forceinline__ X2 mul_pow2(float c, X2 x) { return X2{__fmul2_rn(x.v, make_float2(c, c))}; }
+
+// qsum of collide27_exact.cuh. A leading run of negative terms is summed with
+// its sign turned (the first term costs no addition to 0).
 template <int A, int B, int C>
 __device__ __forceinline__ X2 qsum2(const X2 (&f)[27]) {
-    X2 s = x2(0.0f);
+    X2 s;
+    bool first = true, turned = false;
 #pragma unroll
     for (int q = 0; q < 27; ++q) {
         const int cx = q_cx(q), cy = q_cy(q), cz = q_cz(q);
@@ -81,25 +89,18 @@ __device__ __forceinline__ X2 qsum2(const X2 (&f)[27]) {
         const int pz = C == 0 ? 1 : (C == 2 ? cz * cz : (C == 1 ? cz : 1));
         const int coef = px * py * pz;
         if (coef == 0) continue;
-        s = coef > 0 ? s + f[q] : s - f[q];
+        if (first) {
+            s = f[q];
+            turned = coef < 0;
+            first = false;
+        } else if (turned && coef > 0) {
+            s = f[q] - s;
+            turned = false;
+        } else {
+            s = turned || coef > 0 ? s + f[q] : s - f[q];
+        }
     }
     return s;
-}
-
-// cdot of collide27_exact.cuh: x, y, z components in order, zeros skipped
-__device__ __forceinline__ X2 cdot2x(int q, X2 ux, X2 uy, X2 uz) {
-    const int cx = q_cx(q), cy = q_cy(q), cz = q_cz(q);
-    X2 s = x2(0.0f);
-    bool any = false;
-    if (cx != 0) { s = cx > 0 ? ux : -ux; any = true; }
-    if (cy != 0) { const X2 t = cy > 0 ? uy : -uy; s = any ? s + t : t; any = true; }
-    if (cz != 0) { const X2 t = cz > 0 ? uz : -uz; s = any ? s + t : t; any = true; }
-    return s;
-}
-
-__device__ __forceinline__ X2 feq2x(const Mul2& M, int q, X2 rho, X2 ux, X2 uy, X2 uz, X2 uu) {
-    const X2 cu = M(x2(3.0f), cdot2x(q, ux, uy, uz));
-    return M(M(x2(q_w(q)), rho), ((x2(1.0f) + cu) + M(M(x2(0.5f), cu), cu)) - M(x2(1.5f), uu));
 }
 
 // Collide two fluid cells in place; ok[k] = false: lane k's input was not
@@ -237,104 +238,15 @@ __device__ __forceinline__ void collide27_exact_x2_impl(X2 (&f)[27], const Colli
                        ir);
     }
 
-    const X2 upx[3] = {x2(1.0f), ux, M(ux, ux)};
-    const X2 upy[3] = {x2(1.0f), uy, M(uy, uy)};
-    const X2 upz[3] = {x2(1.0f), uz, M(uz, uz)};
-    // central_to_raw entry R[a][b][c] and raw_to_populations entry fc[q]
-    // (collide27_exact.cuh's loops, one entry per call).
-    X2 R[3][3][3];
-    auto raw = [&](int a, int b, int c) {
-        X2 sum = x2(0.0f);
-        bool first = true;
-#pragma unroll
-        for (int p = 0; p <= a; ++p)
-#pragma unroll
-            for (int qq = 0; qq <= b; ++qq)
-#pragma unroll
-                for (int r = 0; r <= c; ++r) {
-                    if (((p + qq + r) & 1) != 0) continue;
-                    X2 t = x2(float(binom2(a, p) * binom2(b, qq) * binom2(c, r)));
-                    if (a - p > 0) t = M(t, upx[a - p]);
-                    if (b - qq > 0) t = M(t, upy[b - qq]);
-                    if (c - r > 0) t = M(t, upz[c - r]);
-                    t = M(t, K[p][qq][r]);
-                    sum = first ? t : sum + t;
-                    first = false;
-                }
-        R[a][b][c] = sum;
-    };
-    constexpr float inv1[3][3] = {{0.0f, -0.5f, 0.5f}, {1.0f, 0.0f, -1.0f}, {0.0f, 0.5f, 0.5f}};
     X2 fc[27];
-    auto pop = [&](int ix, int iy, int iz) {
-        X2 sum = x2(0.0f);
-        bool first = true;
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float coef = inv1[ix][a] * inv1[iy][b] * inv1[iz][c];
-                    if (coef == 0.0f) continue;
-                    sum = first ? M(x2(coef), R[a][b][c]) : xfma(x2(coef), R[a][b][c], sum);
-                    first = false;
-                }
-        fc[(ix * 3 + iy) * 3 + iz] = sum;
-    };
-    // Populations with cx = 0 read only R[0][.][.] and R[2][.][.], the others
-    // only R[1][.][.] and R[2][.][.]: form them in that order so that R[0]
-    // and R[1] are never live together (fewer registers; same values).
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            raw(0, b, c);
-            raw(2, b, c);
-        }
-#pragma unroll
-    for (int iy = 0; iy < 3; ++iy)
-#pragma unroll
-        for (int iz = 0; iz < 3; ++iz) pop(1, iy, iz);
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) raw(1, b, c);
-#pragma unroll
-    for (int iy = 0; iy < 3; ++iy)
-#pragma unroll
-        for (int iz = 0; iz < 3; ++iz) {
-            pop(0, iy, iz);
-            pop(2, iy, iz);
-        }
-
-    const X2 rho_c = qsum2<0, 0, 0>(fc);
-    const X2 mx_c = qsum2<1, 0, 0>(fc);
-    const X2 my_c = qsum2<0, 1, 0>(fc);
-    const X2 mz_c = qsum2<0, 0, 1>(fc);
-    const X2 rho_cs = rmax2(1e-6f, rho_c);
-    const X2 uxc = div2x(mx_c, rho_cs), uyc = div2x(my_c, rho_cs), uzc = div2x(mz_c, rho_cs);
-    const X2 uu = (M(ux, ux) + M(uy, uy)) + M(uz, uz);
-    const X2 uuc = (M(uxc, uxc) + M(uyc, uyc)) + M(uzc, uzc);
-#pragma unroll
-    for (int q = 0; q < 27; ++q)
-        fc[q] = fc[q] + (feq2x(M, q, rho_safe, ux, uy, uz, uu) - feq2x(M, q, rho_cs, uxc, uyc, uzc, uuc));
-
+    central_to_populations(M, K, ux, uy, uz, fc);
+    const X2 rho_cs = rmax2(1e-6f, carried_sum<0>(fc));
+    const X2 uxc = div2x(carried_sum<1>(fc), rho_cs), uyc = div2x(carried_sum<2>(fc), rho_cs),
+             uzc = div2x(carried_sum<3>(fc), rho_cs);
+    conserve(M, fc, rho_safe, ux, uy, uz, rho_cs, uxc, uyc, uzc, f);
     if (forced0 || forced1) {
-        const float inv_cs2 = 1.0f / kCs2f;
-        const float inv_cs4 = inv_cs2 * inv_cs2;
-        const X2 oc = rclamp2(omega_off, 0.0f, 1.999f);
-        const X2 pref = rmax2(0.0f, x2(1.0f) - M(x2(0.5f), oc));
-        const X2 u_force = (M(ux, fx) + M(uy, fy)) + M(uz, fz);
-#pragma unroll
-        for (int q = 0; q < 27; ++q) {
-            const X2 cu = cdot2x(q, ux, uy, uz);
-            const X2 c_force = cdot2x(q, fx, fy, fz);
-            const X2 g = fc[q] + M(M(pref, x2(q_w(q))), M(c_force - u_force, x2(inv_cs2)) + M(M(cu, c_force), x2(inv_cs4)));
-            f[q] = sel2(forced0, forced1, g, fc[q]);
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < 27; ++q) f[q] = fc[q];
+        const X2 pref = rmax2(0.0f, x2(1.0f) - M(x2(0.5f), rclamp2(omega_off, 0.0f, 1.999f)));
+        guo(M, pref, ux, uy, uz, fx, fy, fz, f, [&](int q, X2 v) { f[q] = sel2(forced0, forced1, v, f[q]); });
     }
 }
 
