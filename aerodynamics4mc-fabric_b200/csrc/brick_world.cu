@@ -737,6 +737,79 @@ void adopt_next(Brick& b, Next& next) {
     }
 }
 
+// Inputs of a brick's call, read from its dynamic buffer `buffer`.
+FillArgs fill_args(const World& w, const Coord& c, const Brick& b, int buffer) {
+    FillArgs fa{};
+    fa.n = w.brick_size;
+    fa.st = static_dev(b);
+    fa.flow = b.mem.flow[buffer];
+    fa.air = b.mem.air[buffer];
+    if (b.reference) {
+        fa.ref_flow = b.mem.ref_flow;
+        fa.ref_air = b.mem.ref_air;
+        fa.exposed = exposed_mask(w, c);
+    }
+    fa.ref_layers = std::max(1, std::min(kBoundaryReferenceLayers, fa.n));
+    fa.source_denominator = kSourceDenominator;
+    return fa;
+}
+
+// Arguments of a brick's dynamic refresh into buffer dst, with the static
+// constraints (sync_from_context's; the temperature source is the caller's).
+SyncArgs sync_args(const Service& svc, const World& w, const Brick& b, int dst, int surface_from) {
+    SyncArgs a{};
+    a.cells = (long long)w.brick_size * w.brick_size * w.brick_size;
+    a.flow = b.mem.flow[dst];
+    a.air = b.mem.air[dst];
+    a.surface = b.mem.surface[dst];
+    a.surface_src = b.mem.surface[surface_from];
+    if (b.stat) a.st = static_dev(b);
+    a.flag = svc.d_flags + b.flag_slot;
+    return a;
+}
+
+// Bricks whose call needs none of step_brick's rare paths: the same mask and
+// forcing as the last call of a live context, in the classic solver modes.
+// They step together (world_step_batch) after the tick's other bricks.
+struct TogetherBrick {
+    Coord coord;
+    Brick* brick;
+};
+bool steps_together(const World& w, const Brick& b) {
+    return !experimental(w) && b.context != 0 && b.stat && b.has_dynamic && !b.forcing_dirty && !b.geometry_dirty &&
+           !b.pending_reinit && b.stepped_context == b.context && b.stepped_version == b.static_version;
+}
+
+bool step_together(Service& svc, World& w, const std::vector<TogetherBrick>& bricks) {
+    ModeScope scope(w.solver_mode);
+    const int n = w.brick_size;
+    std::vector<WorldStepJob> jobs;
+    jobs.reserve(bricks.size());
+    for (const TogetherBrick& t : bricks) {
+        w.packet_build_steps++;
+        w.d3q27_steps++;
+        t.brick->compact_active = false;
+        jobs.push_back(WorldStepJob{find_context(t.brick->context), fill_args(w, t.coord, *t.brick, t.brick->cur),
+                                    sync_args(svc, w, *t.brick, 1 - t.brick->cur, t.brick->cur)});
+    }
+    if (!world_step_batch(jobs)) {
+        set_sim_error("brick_step_actual: aero_lbm_step_rect failed at " + coord_text(bricks.front().coord) + ": " + last_error());
+        for (const TogetherBrick& t : bricks) release_context(svc, *t.brick);
+        return false;
+    }
+    for (const TogetherBrick& t : bricks) {
+        Brick& b = *t.brick;
+        b.cur = 1 - b.cur;
+        expect_flag(svc, b);
+        b.constrained_version = b.static_version;
+        b.stale = false;
+        update_shell(w, t.coord, b);
+        b.pending_patch_cells.clear();
+        b.pending_reinit = b.geometry_dirty = b.forcing_dirty = false;
+    }
+    return true;
+}
+
 // step_brick_actual (simulation_bridge.cpp:1706-1832)
 bool step_brick(Service& svc, World& w, const Coord& c, Brick& b, Next& next, std::vector<Fallback>& fallbacks) {
     ModeScope scope(w.solver_mode);
@@ -755,21 +828,10 @@ bool step_brick(Service& svc, World& w, const Coord& c, Brick& b, Next& next, st
     const bool had_context = b.context != 0;
     if (b.context == 0) b.context = svc.next_context_key--;
 
-    FillArgs fa{};
-    fa.n = n;
-    fa.st = static_dev(b);
-    fa.flow = b.mem.flow[next.buffer];
-    fa.air = b.mem.air[next.buffer];
-    if (b.reference) {
-        fa.ref_flow = b.mem.ref_flow;
-        fa.ref_air = b.mem.ref_air;
-        fa.exposed = exposed_mask(w, c);
-    }
-    fa.ref_layers = std::max(1, std::min(kBoundaryReferenceLayers, n));
-    fa.source_denominator = kSourceDenominator;
+    const FillArgs fa = fill_args(w, c, b, next.buffer);
     // the mask comes from the static fields alone: unchanged since this
     // context's last step, the step keeps its pull classification
-    const DeviceFill fill{fill_launch, &fa,
+    const DeviceFill fill{fill_launch, const_cast<FillArgs*>(&fa),
                           had_context && b.stepped_context == b.context && b.stepped_version == b.static_version};
 
     bool step_ok = false, compact_ok = false, have_summary = false, fill_stepped = false;
@@ -935,6 +997,7 @@ bool step_world(Service& svc, long long wkey, World& w, int steps) {
             return false;
         }
         std::vector<Fallback> fallbacks;
+        std::vector<TogetherBrick> together;
         SnapshotCache cache;
         for (auto& [c, b] : w.bricks) {
             if (!solver_active(w, b) || !b.has_dynamic) continue;
@@ -945,6 +1008,10 @@ bool step_world(Service& svc, long long wkey, World& w, int steps) {
                 continue;
             }
             if (!ensure_dynamic(svc, w, b) || !device_ready(svc, w, b)) return false;
+            if (!seed && steps_together(w, b) && world_step_ready(find_context(b.context), n, n, n)) {
+                together.push_back(TogetherBrick{c, &b});
+                continue;
+            }
             const bool bootstrap = seed || b.context == 0;
             Next next{b.cur, nullptr, b.nonzero};
             if (seed || bootstrap) {
@@ -978,6 +1045,7 @@ bool step_world(Service& svc, long long wkey, World& w, int steps) {
             if (!step_brick(svc, w, c, b, next, fallbacks)) all_ok = false;
             b.pending_reinit = b.geometry_dirty = b.forcing_dirty = false;
         }
+        if (!together.empty() && !step_together(svc, w, together)) all_ok = false;
         if (!resolve_flags(svc)) return false;
         // a step whose output came back all zero after its static fields
         // changed keeps the state it started from (zero_output_fallback)
@@ -1611,6 +1679,19 @@ AERO_LBM_B200_EXPORT int aero_lbm_simulation_copy_brick_world_packed_flow_atlas(
             set_sim_error("simulation_copy_brick_world_packed_flow_atlas extract failed: "
                           "extract_flow_atlas: no initialized context of these dimensions");
             return 0;
+        }
+        bool done = false;
+        if (!world_atlas(*ctx, pa, &done)) {
+            set_sim_error(std::string("simulation_copy_brick_world_packed_flow_atlas extract failed: ") + last_error());
+            return 0;
+        }
+        if (done) {
+            if (!cuda_ok(cudaStreamSynchronize(s), "publish atlas")) {
+                set_sim_error(std::string("simulation_copy_brick_world_packed_flow_atlas: ") + last_error());
+                return 0;
+            }
+            std::memcpy(out_packed_flow, svc->h_atlas, (size_t)samples * 8);
+            return 1;
         }
         if ((size_t)samples > svc->atlas_cap) {
             if (svc->d_atlas) cudaFree(svc->d_atlas);

@@ -230,19 +230,10 @@ __device__ __forceinline__ void fused_transport(const IpArgs& a, int x, int y, i
                                         fused_sv, reinterpret_cast<unsigned char*>(fused_sv + 9 * W));
 }
 
-template <class S, bool kExact, int kParity, bool kTransport>
-__global__ void __launch_bounds__(128) step_ip_kernel(typename S::T* __restrict__ f, IpArgs a) {
-    const PadGeom G = a.g;
-    int x, y, z;
-    long long cell;
-    const bool in_line = line_cell(G, x, y, z, cell);
-    float tn[1] = {0.0f};
-    if (kTransport) {
-        const int z_begin = blockIdx.x * blockDim.x;
-        const int zs[1] = {z};
-        fused_transport<1>(a, x, y, z_begin, min((int)blockDim.x, G.nz - z_begin), zs, tn);
-    }
-    if (!in_line) return;
+// One cell of the step. tn: the cell's temperature where the caller computed it.
+template <class S, bool kExact, int kParity>
+__device__ __forceinline__ void step_ip_cell(typename S::T* __restrict__ f, const IpArgs& a, const PadGeom& G, long long cell,
+                                             int x, int y, int z, const float* tn) {
     const uint32_t w = a.flags_prev[cell];
     if (w & kFlagSelfSolid) {  // memory of a solid cell is link storage; transitions run separately
         record_u(a.cur, cell, 0.0f, 0.0f, 0.0f);
@@ -258,7 +249,7 @@ __global__ void __launch_bounds__(128) step_ip_kernel(typename S::T* __restrict_
         fl[q] = S::load(f + (d * G.pcells + c), q, a.sc);
     }
     if (a.obstacle_cur[cell]) record_u(a.cur, cell, 0.0f, 0.0f, 0.0f);
-    if (!a.obstacle_cur[cell] && !collide_cell<kExact>(fl, a.cp, a.cur, a.force, cell, x, y, z, kTransport ? tn : nullptr)) {
+    if (!a.obstacle_cur[cell] && !collide_cell<kExact>(fl, a.cp, a.cur, a.force, cell, x, y, z, tn)) {
         reseed_push<S>(f, a, cell, x, y, z, kParity);
         return;
     }
@@ -268,6 +259,22 @@ __global__ void __launch_bounds__(128) step_ip_kernel(typename S::T* __restrict_
         outgoing_slot(o, own, q, kParity, c, d);
         S::store(f + (d * G.pcells + c), q, fl[q], a.sc);
     }
+}
+
+template <class S, bool kExact, int kParity, bool kTransport>
+__global__ void __launch_bounds__(128) step_ip_kernel(typename S::T* __restrict__ f, IpArgs a) {
+    const PadGeom G = a.g;
+    int x, y, z;
+    long long cell;
+    const bool in_line = line_cell(G, x, y, z, cell);
+    float tn[1] = {0.0f};
+    if (kTransport) {
+        const int z_begin = blockIdx.x * blockDim.x;
+        const int zs[1] = {z};
+        fused_transport<1>(a, x, y, z_begin, min((int)blockDim.x, G.nz - z_begin), zs, tn);
+    }
+    if (!in_line) return;
+    step_ip_cell<S, kExact, kParity>(f, a, G, cell, x, y, z, kTransport ? tn : nullptr);
 }
 
 // Loads and stores of two cells' populations of one direction: at two
@@ -758,6 +765,21 @@ __global__ void __launch_bounds__(128) init_ip_kernel(typename S::T* __restrict_
     ip_push<S>(f, a, G, o, own, 0, fl);
 }
 
+// Macro output of one cell's streamed state (what the next step would pull).
+template <class S, bool kExact>
+__device__ __forceinline__ void macro_ip_cell(const typename S::T* __restrict__ f, const IpArgs& a, const PadGeom& G,
+                                              long long cell, int x, int y, int z, float scale, float (&o4)[4]) {
+    const uint32_t w = a.flags_prev[cell];
+    o4[0] = o4[1] = o4[2] = o4[3] = 0.0f;
+    if (w & kFlagSelfSolid) return;
+    const int own = pad_index(G, x, y, z);
+    const NeighbourOffsets o = neighbour_offsets(G, x, y, z);
+    float fl[27];
+    ip_pull<S>(f, a, G, o, own, w, a.parity, fl);
+    if (kExact) exact::macro_out_exact(fl, false, scale, o4);
+    else macro_out(fl, false, scale, o4);
+}
+
 // Macro output of the streamed state (what the next step would pull), with
 // write_output / strided-extract semantics. Read-only.
 template <class S, bool kExact>
@@ -772,16 +794,8 @@ __global__ void output_ip_kernel(const typename S::T* __restrict__ f, IpArgs a, 
     const int x = min(G.nx - 1, b.ox + ax * b.stride), y = min(G.ny - 1, b.oy + ay * b.stride),
               z = min(G.nz - 1, b.oz + az * b.stride);
     const long long cell = ((long long)x * G.ny + y) * G.nz + z;
-    const uint32_t w = a.flags_prev[cell];
-    float o4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (!(w & kFlagSelfSolid)) {
-        const int own = pad_index(G, x, y, z);
-        const NeighbourOffsets o = neighbour_offsets(G, x, y, z);
-        float fl[27];
-        ip_pull<S>(f, a, G, o, own, w, a.parity, fl);
-        if (kExact) exact::macro_out_exact(fl, false, scale, o4);
-        else macro_out(fl, false, scale, o4);
-    }
+    float o4[4];
+    macro_ip_cell<S, kExact>(f, a, G, cell, x, y, z, scale, o4);
     float* dst = out + i * out_ch;
     dst[0] = o4[0]; dst[1] = o4[1]; dst[2] = o4[2]; dst[3] = o4[3];
     for (int c = 4; c < out_ch; ++c) dst[c] = 0.0f;

@@ -29,6 +29,7 @@
 #include "halo.cuh"
 #include "runtime_internal.h"
 #include "thermal.cuh"
+#include "world_step.cuh"
 
 namespace aero {
 
@@ -489,6 +490,7 @@ bool Context::allocate(int nx_, int ny_, int nz_) {
     f_ready = false;
     force_valid = false;
     slot = 0;
+    slots_match = false;
     cur = 0;
     step_counter = 0;
     return true;
@@ -699,6 +701,7 @@ static bool choose_layout(Context& ctx, const FaceParams& face, const float* pac
 // Build the pull classification of `slot` for faces `face` and keep a device
 // copy of the faces for the kernels that stream with this slot.
 static bool classify(Context& ctx, int slot, const FaceParams& face, const BrickDims& d, cudaStream_t s) {
+    ctx.slots_match = false;
     ctx.h_face[slot] = face;
     if (!cuda_ok(cudaMemcpyAsync(ctx.d_face[slot], &ctx.h_face[slot], sizeof(FaceParams), cudaMemcpyHostToDevice, s),
                  "upload faces")) return false;
@@ -735,6 +738,29 @@ static float thermal_diffusivity() {
     if (!heated_cavity()) return kThermalDiffusivity;
     const float pr = std::max(1.0e-6f, finite_or(g_bench.prandtl_number, 0.71f));
     return base_nu_shear() / pr;
+}
+
+// The temperature update of a call that collides with mask `obstacle`.
+static ThermalArgs thermal_args(const Context& ctx, const uint8_t* obstacle, const CollideParams& cp) {
+    ThermalArgs ta{};
+    ta.nx = ctx.nx; ta.ny = ctx.ny; ta.nz = ctx.nz; ta.cells = ctx.cells;
+    ta.t = ctx.temperature;
+    ta.t_next = ctx.temperature_next;
+    ta.u = ctx.u_last;
+    ta.obstacle = obstacle;
+    ta.source = bench_flag(AERO_LBM_BENCHMARK_FLAG_DISABLE_INTERNAL_THERMAL_SOURCE) ? nullptr : ctx.thermal_source;
+    ta.alpha = thermal_diffusivity();
+    ta.faces = current_thermal_faces();
+    // thermal_bfecc_active (jni.cpp:871-873); outside benchmark mode the
+    // update also runs every other call with dt = 2 and a local eddy
+    // diffusivity (effective_thermal_dt, effective_local_thermal_diffusivity)
+    ta.bfecc = (!bench_active() || heated_cavity()) ? 1 : 0;
+    ta.scratch = ctx.temperature_scratch;
+    ta.dt = bench_active() ? 1.0f : 2.0f;
+    ta.turbulent = (!bench_active() && cp.enable_sgs) ? 1 : 0;
+    ta.sgs_c2 = cp.sgs_c2;
+    ta.nu0 = clamp_nu(kRuntimeMolecularNu0);
+    return ta;
 }
 
 // One step of a context. packet may be null (cached step); out may be null.
@@ -840,12 +866,15 @@ static bool step_context_body(Context& ctx, const float* packet, float* out, flo
         }
         if (host_packet && !cuda_ok(cudaEventRecord(ctx.copy_done, s), "copy event")) return false;
         if (same_mask) {
+            // both slots hold the same classification from the first such call on
             ctx.h_face[new_slot] = face_now;
-            if (!cuda_ok(cudaMemcpyAsync(ctx.d_face[new_slot], ctx.d_face[ctx.slot], sizeof(FaceParams), cudaMemcpyDeviceToDevice, s),
-                         "copy faces") ||
-                !cuda_ok(cudaMemcpyAsync(ctx.flags[new_slot], ctx.flags[ctx.slot], (size_t)ctx.cells * sizeof(uint32_t),
-                                         cudaMemcpyDeviceToDevice, s), "copy classification"))
+            if (!ctx.slots_match &&
+                (!cuda_ok(cudaMemcpyAsync(ctx.d_face[new_slot], ctx.d_face[ctx.slot], sizeof(FaceParams), cudaMemcpyDeviceToDevice, s),
+                          "copy faces") ||
+                 !cuda_ok(cudaMemcpyAsync(ctx.flags[new_slot], ctx.flags[ctx.slot], (size_t)ctx.cells * sizeof(uint32_t),
+                                          cudaMemcpyDeviceToDevice, s), "copy classification")))
                 return false;
+            ctx.slots_match = true;
         } else if (!classify(ctx, new_slot, face_now, d, s)) {
             return false;
         }
@@ -877,24 +906,7 @@ static bool step_context_body(Context& ctx, const float* packet, float* out, flo
         }
         // should_update_temperature (jni.cpp:2191-2196): every other call in runtime mode
         const bool update = bench_active() || ctx.step_counter % 2 == 0;
-        ThermalArgs ta{};
-        ta.nx = ctx.nx; ta.ny = ctx.ny; ta.nz = ctx.nz; ta.cells = ctx.cells;
-        ta.t = ctx.temperature;
-        ta.t_next = ctx.temperature_next;
-        ta.u = ctx.u_last;
-        ta.obstacle = ctx.obstacle[new_slot];
-        ta.source = bench_flag(AERO_LBM_BENCHMARK_FLAG_DISABLE_INTERNAL_THERMAL_SOURCE) ? nullptr : ctx.thermal_source;
-        ta.alpha = thermal_diffusivity();
-        ta.faces = current_thermal_faces();
-        // thermal_bfecc_active (jni.cpp:871-873); outside benchmark mode the
-        // update also runs every other call with dt = 2 and a local eddy
-        // diffusivity (effective_thermal_dt, effective_local_thermal_diffusivity)
-        ta.bfecc = (!bench_active() || heated_cavity()) ? 1 : 0;
-        ta.scratch = ctx.temperature_scratch;
-        ta.dt = bench_active() ? 1.0f : 2.0f;
-        ta.turbulent = (!bench_active() && cp.enable_sgs) ? 1 : 0;
-        ta.sgs_c2 = cp.sgs_c2;
-        ta.nu0 = clamp_nu(kRuntimeMolecularNu0);
+        const ThermalArgs ta = thermal_args(ctx, ctx.obstacle[new_slot], cp);
         // The first-order branch runs inside the in-place step kernel
         // (thermal_fused.cuh) once the context has stepped: the state is
         // swapped here, the kernel reads the old one and writes the new one.
@@ -1021,6 +1033,105 @@ static bool step_context_body(Context& ctx, const float* packet, float* out, flo
     if (out) return read_output(ctx, 1, g_cfg.output_channels, scale, out);
     if (have_packet && host_packet && !cuda_ok(cudaEventSynchronize(ctx.copy_done), "wait for the packet copy")) return false;
     return true;
+}
+
+void record_timing(double copy_ms, double solver_ms, double readback_ms, double total_ms, bool cached);
+
+bool world_step_ready(const Context* c, int nx, int ny, int nz) {
+    if (!c || !c->initialized || !c->has_inputs || c->nx != nx || c->ny != ny || c->nz != nz) return false;
+    if (c->layout != 1 || c->ip_variant != kIpF32Exact || c->pending_slot >= 0 || c->fill_pending || !c->solid_f) return false;
+    if (bench_active() || g_realtime_solver_mode == AERO_LBM_REALTIME_SOLVER_D3Q27_FP16_INPLACE_EXPERIMENTAL) return false;
+    if (!g_cfg.initialized || g_cfg.input_channels <= kChStateTemp) return false;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev != c->device) return false;
+    const FaceParams face = current_face_params();
+    if (std::memcmp(&face, &c->face_prev, sizeof(FaceParams)) != 0 || !inplace_faces_ok(face)) return false;
+    const CollideParams cp = current_collide_params();
+    const bool thermal = g_thermal_mode == 1 || (g_thermal_mode == -1 && cp.enable_buoyancy);
+    return cp.runtime_terms && (cp.fan_beta <= 0.0f || c->fan_mask) && (!thermal || c->u_last);
+}
+
+// The passes of step_context_body for these calls, in its order, each over
+// all bricks (the bricks share nothing between their calls; the halo
+// exchange before them and the refresh flags after them are the caller's).
+bool world_step_batch(const std::vector<WorldStepJob>& jobs) {
+    if (jobs.empty()) return true;
+    const auto t0 = Clock::now();
+    clear_error();
+    cudaStream_t s = current_stream();
+    const FaceParams face = current_face_params();
+    CollideParams cp = current_collide_params();
+    const bool thermal = g_thermal_mode == 1 || (g_thermal_mode == -1 && cp.enable_buoyancy);
+    const unsigned fill_faces = fill_face_mask(face);
+    for (size_t at = 0; at < jobs.size(); at += kWorldChunk) {
+        const size_t n = std::min<size_t>(kWorldChunk, jobs.size() - at);
+        std::vector<WorldInputs> in(n);
+        std::vector<WorldStep> step[2], post(n);
+        std::vector<WorldOutput> out(n);
+        std::vector<ThermalArgs> heat;
+        for (size_t i = 0; i < n; ++i) {
+            const WorldStepJob& job = jobs[at + i];
+            Context& c = *job.ctx;
+            c.thermal = thermal;
+            cp.nx = c.nx;
+            cp.ny = c.ny;
+            cp.nz = c.nz;
+            cp.step = c.step_counter;
+            const int from = c.slot, to = 1 - c.slot;
+            in[i] = WorldInputs{job.fill, c.fields(to), ThermalNudgeArgs{}, job.sync.flag};
+            if (thermal) {
+                in[i].nudge = ThermalNudgeArgs{c.nx, c.ny, c.nz, c.temperature, c.obstacle[to], c.ref_temperature, cp.state_nudge};
+                if (c.step_counter % 2 == 0) {
+                    // runtime mode updates the temperature every other call (BFECC)
+                    heat.push_back(thermal_args(c, c.obstacle[to], cp));
+                    std::swap(c.temperature, c.temperature_scratch);
+                }
+            }
+            // the mask is unchanged: both slots hold (or now take) the same classification
+            if (!c.slots_match) {
+                if (!cuda_ok(cudaMemcpyAsync(c.d_face[to], c.d_face[from], sizeof(FaceParams), cudaMemcpyDeviceToDevice, s), "copy faces") ||
+                    !cuda_ok(cudaMemcpyAsync(c.flags[to], c.flags[from], (size_t)c.cells * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s),
+                             "copy classification"))
+                    return false;
+                c.slots_match = true;
+            }
+            c.h_face[to] = face;
+            WorldStep st{static_cast<float*>(c.ip), ip_args(c, from, to, cp)};
+            st.a.parity = c.parity;
+            step[c.parity & 1].push_back(st);
+            c.parity ^= 1;
+            st.a = ip_args(c, to, to, cp);
+            st.a.parity = c.parity;
+            st.a.fill_faces = fill_faces;
+            post[i] = st;
+            out[i] = WorldOutput{st.f, st.a, job.sync};
+            out[i].sync.temperature = c.temperature;
+            c.slot = to;
+            c.face_prev = face;
+            c.step_counter += 1;
+            c.force_valid = false;
+        }
+        bool ok = cuda_ok(launch_world_inputs(in.data(), (int)n, s), "world inputs");
+        if (ok && !heat.empty()) ok = cuda_ok(launch_bfecc_batch(heat.data(), (int)heat.size(), s), "world temperature");
+        for (int p = 0; p < 2 && ok; ++p)
+            if (!step[p].empty()) ok = cuda_ok(launch_world_step(step[p].data(), (int)step[p].size(), p, s), "world step");
+        if (ok && fill_faces) ok = cuda_ok(launch_world_face_fill(post.data(), (int)n, s), "world face pre-fill");
+        if (ok) ok = cuda_ok(launch_world_output(out.data(), (int)n, s), "world output");
+        if (!ok) return false;
+    }
+    const double ms = ms_since(t0) / (double)jobs.size();
+    for (size_t i = 0; i < jobs.size(); ++i) record_timing(0.0, 0.0, 0.0, ms, false);
+    return true;
+}
+
+bool world_atlas(Context& ctx, const bw::PublishArgs& p, bool* done) {
+    *done = ctx.layout == 1 && ctx.ip_variant == kIpF32Exact;
+    if (!*done) return true;
+    cudaStream_t s = current_stream();
+    if (!join_fill(ctx, s)) return false;
+    IpArgs a = ip_args(ctx, ctx.slot, ctx.slot, current_collide_params());
+    a.parity = ctx.parity;
+    return cuda_ok(launch_world_atlas(static_cast<const float*>(ctx.ip), a, p, s), "world atlas");
 }
 
 bool output_device(Context& ctx, OutBox box, int out_ch, float scale, float* dev_out) {
@@ -1610,6 +1721,7 @@ AERO_LBM_B200_EXPORT int aero_lbm_shift_context(int grid_size, long long key, in
     if (!shift_scalar(c->ref_p[slot]) || !shift_scalar(c->ref_ux) || !shift_scalar(c->ref_uy) || !shift_scalar(c->ref_uz) ||
         !shift_scalar(c->ref_temperature) || !shift_scalar(c->thermal_source))
         return 0;
+    c->slots_match = false;
     if (!cuda_ok(launch_build_flags(c->obstacle[slot], d, c->h_face[slot], c->flags[slot], s), "shift flags")) return 0;
     if (c->layout == 1) {
         v.flags = c->flags[slot];

@@ -4,9 +4,11 @@
 #include <cstdint>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include <cuda_runtime.h>
 
+#include "brick_world.cuh"
 #include "d3q27_kernels.cuh"
 
 namespace aero {
@@ -91,6 +93,7 @@ struct Context {
     int shell_layers = 0;
     float shell_relax = 0.0f;
     int slot = 0;
+    bool slots_match = false;  // flags and d_face of the two slots hold the same classification
     bool allocated = false;
     bool initialized = false;
     bool has_inputs = false;
@@ -141,6 +144,24 @@ bool step_context(Context& ctx, const float* packet, float* out, float scale, bo
 // aero_lbm_step_rect for a call whose inputs `fill` builds on the device:
 // the same context lookup / creation, checks and timing record; no output.
 bool step_rect_device(long long key, int nx, int ny, int nz, const DeviceFill& fill);
+// One brick of a world's tick stepped with the others (world_step.cuh): its
+// inputs, and the dynamic refresh after its call (sync.temperature is set by
+// the step).
+struct WorldStepJob {
+    Context* ctx;
+    bw::FillArgs fill;
+    bw::SyncArgs sync;
+};
+// Whether a context's next call with device-built inputs and an unchanged
+// mask is one world_step_batch takes: an in-place FP32 reference-order context
+// in runtime mode, stepped before, with nothing staged or pending.
+bool world_step_ready(const Context* ctx, int nx, int ny, int nz);
+// The calls of step_rect_device (mask unchanged) and the flow output of each
+// job's context, launched over all jobs (one size) together.
+bool world_step_batch(const std::vector<WorldStepJob>& jobs);
+// A packed atlas straight from a context's populations; false in *done when
+// the context's layout has no such pass.
+bool world_atlas(Context& ctx, const bw::PublishArgs& p, bool* done);
 bool read_output(Context& ctx, int stride, int out_ch, float scale, float* host_out);
 // Per-brick FP16 deviation scale for a brick whose speed stays below umax.
 float fp16_scale_for_speed(float umax);

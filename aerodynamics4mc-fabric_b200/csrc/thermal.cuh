@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include "d3q27_kernels.cuh"
+#include "lattice.cuh"
 
 namespace aero {
 
@@ -88,6 +89,33 @@ struct ThermalNudgeArgs {
     float nudge;                // 0.08
 };
 cudaError_t launch_thermal_reference_nudge(const ThermalNudgeArgs& a, cudaStream_t s);
+// (in units built without multiply-add contraction)
+__device__ __forceinline__ void thermal_nudge_cell(const ThermalNudgeArgs& a, long long cell) {
+    auto clamp1 = [](float v) {
+        const float m = (-1.0f < v) ? v : -1.0f;
+        return (m < 1.0f) ? m : 1.0f;
+    };
+    if (a.obstacle[cell]) {
+        a.t[cell] = 0.0f;
+        return;
+    }
+    int x, y, z;
+    cell_xyz32(cell, a.ny, a.nz, x, y, z);
+    const int d = min(min(min(x, y), min(z, a.nx - 1 - x)), min(a.ny - 1 - y, a.nz - 1 - z));
+    if (d >= 8) return;
+    const float eta = (float)(8 - d) / 8.0f;
+    const float n = a.nudge * eta * eta;
+    if (n <= 0.0f) return;
+    const float rt = clamp1(a.ref_t[cell]);
+    const float keep = 1.0f - n;
+    a.t[cell] = clamp1(a.t[cell] * keep + rt * n);
+}
+
+// Bricks one launch of a world's tick takes (their arguments travel in the
+// launch's parameter space, 32764 bytes at most).
+constexpr int kWorldChunk = 32;
+// The BFECC update of n <= kWorldChunk bricks of one size: three launches.
+cudaError_t launch_bfecc_batch(const ThermalArgs* args, int n, cudaStream_t s);
 
 // First call of a context: the state and the velocity the first update
 // advects with (initialize_distributions, jni.cpp:1752-1781). benchmark: a

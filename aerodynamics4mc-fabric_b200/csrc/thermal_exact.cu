@@ -255,9 +255,7 @@ __device__ __forceinline__ bool th_line_cell(const ThermalArgs& a, int& x, int& 
 }
 
 // scratch = A_-(T)
-__global__ void __launch_bounds__(128) bfecc_forward_kernel(const __grid_constant__ ThermalArgs a) {
-    int x, y, z, cell;
-    if (!th_line_cell(a, x, y, z, cell)) return;
+__device__ __forceinline__ void bfecc_forward(const ThermalArgs& a, int x, int y, int z, int cell) {
     if (a.obstacle[cell]) {
         a.scratch[cell] = 0.0f;
         return;
@@ -268,9 +266,7 @@ __global__ void __launch_bounds__(128) bfecc_forward_kernel(const __grid_constan
 }
 
 // next = clamp(T + (T - A_+(scratch)) / 2)
-__global__ void __launch_bounds__(128) bfecc_correct_kernel(const __grid_constant__ ThermalArgs a) {
-    int x, y, z, cell;
-    if (!th_line_cell(a, x, y, z, cell)) return;
+__device__ __forceinline__ void bfecc_correct(const ThermalArgs& a, int x, int y, int z, int cell) {
     if (a.obstacle[cell]) {
         a.t_next[cell] = 0.0f;
         return;
@@ -283,9 +279,7 @@ __global__ void __launch_bounds__(128) bfecc_correct_kernel(const __grid_constan
 }
 
 // scratch = clamp(clamp(A_-(next), local bounds of T) + dt (alpha lap T + s))
-__global__ void __launch_bounds__(128) bfecc_final_kernel(const __grid_constant__ ThermalArgs a) {
-    int x, y, z, cell;
-    if (!th_line_cell(a, x, y, z, cell)) return;
+__device__ __forceinline__ void bfecc_final(const ThermalArgs& a, int x, int y, int z, int cell) {
     if (a.obstacle[cell]) {
         a.scratch[cell] = 0.0f;
         return;
@@ -336,24 +330,36 @@ __global__ void __launch_bounds__(128) bfecc_final_kernel(const __grid_constant_
     a.scratch[cell] = exact::rclamp(adv + dt * (alpha * lap + src - cooling * adv), -1.0f, 1.0f);
 }
 
+// The three passes on one brick, and (a block per 128 cells of brick
+// blockIdx.y) on several bricks of one size.
+template <int kPass>
+__device__ __forceinline__ void bfecc_pass(const ThermalArgs& a, int x, int y, int z, int cell) {
+    if (kPass == 0) bfecc_forward(a, x, y, z, cell);
+    else if (kPass == 1) bfecc_correct(a, x, y, z, cell);
+    else bfecc_final(a, x, y, z, cell);
+}
+template <int kPass>
+__global__ void __launch_bounds__(128) bfecc_kernel(const __grid_constant__ ThermalArgs a) {
+    int x, y, z, cell;
+    if (th_line_cell(a, x, y, z, cell)) bfecc_pass<kPass>(a, x, y, z, cell);
+}
+struct BfeccJobs {
+    ThermalArgs a[kWorldChunk];
+};
+template <int kPass>
+__global__ void __launch_bounds__(128) bfecc_batch_kernel(const __grid_constant__ BfeccJobs jobs) {
+    const ThermalArgs& a = jobs.a[blockIdx.y];
+    const int cell = blockIdx.x * blockDim.x + threadIdx.x;
+    if (cell >= a.cells) return;
+    int x, y, z;
+    cell_xyz32(cell, a.ny, a.nz, x, y, z);
+    bfecc_pass<kPass>(a, x, y, z, cell);
+}
+
 __global__ void thermal_reference_nudge_kernel(ThermalNudgeArgs a) {
     const long long cells = (long long)a.nx * a.ny * a.nz;
     const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (cell >= cells) return;
-    if (a.obstacle[cell]) {
-        a.t[cell] = 0.0f;
-        return;
-    }
-    int x, y, z;
-    cell_xyz32(cell, a.ny, a.nz, x, y, z);
-    const int d = min(min(min(x, y), min(z, a.nx - 1 - x)), min(a.ny - 1 - y, a.nz - 1 - z));
-    if (d >= 8) return;
-    const float eta = (float)(8 - d) / 8.0f;
-    const float n = a.nudge * eta * eta;
-    if (n <= 0.0f) return;
-    const float rt = exact::rclamp(a.ref_t[cell], -1.0f, 1.0f);
-    const float keep = 1.0f - n;
-    a.t[cell] = exact::rclamp(a.t[cell] * keep + rt * n, -1.0f, 1.0f);
+    if (cell < cells) thermal_nudge_cell(a, cell);
 }
 
 // The staged z-pairs of one thread (e = 0: pair tid, e = 1: pair tid + 128
@@ -811,11 +817,11 @@ cudaError_t launch_thermal_update(const ThermalArgs& a, cudaStream_t s) {
     if (a.bfecc) {
         const int block = a.nz >= 128 ? 128 : ((a.nz + 31) / 32) * 32;
         const dim3 grid((unsigned)((a.nz + block - 1) / block), (unsigned)a.ny, (unsigned)a.nx);
-        bfecc_forward_kernel<<<grid, block, 0, s>>>(a);
+        bfecc_kernel<0><<<grid, block, 0, s>>>(a);
         count_launch();
-        bfecc_correct_kernel<<<grid, block, 0, s>>>(a);
+        bfecc_kernel<1><<<grid, block, 0, s>>>(a);
         count_launch();
-        bfecc_final_kernel<<<grid, block, 0, s>>>(a);
+        bfecc_kernel<2><<<grid, block, 0, s>>>(a);
         count_launch();
         return cudaGetLastError();
     }
@@ -826,6 +832,20 @@ cudaError_t launch_thermal_update(const ThermalArgs& a, cudaStream_t s) {
                                               : launch_pdl(thermal_update_kernel<false>, grid, dim3(kMTZ, kMY), 0, s, ap);
     count_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+cudaError_t launch_bfecc_batch(const ThermalArgs* args, int n, cudaStream_t s) {
+    if (n < 1 || n > kWorldChunk || args[0].cells >= (1LL << 31)) return cudaErrorInvalidValue;
+    BfeccJobs jobs;
+    for (int i = 0; i < n; ++i) jobs.a[i] = args[i];
+    const dim3 grid((unsigned)((args[0].cells + 127) / 128), (unsigned)n);
+    bfecc_batch_kernel<0><<<grid, 128, 0, s>>>(jobs);
+    count_launch();
+    bfecc_batch_kernel<1><<<grid, 128, 0, s>>>(jobs);
+    count_launch();
+    bfecc_batch_kernel<2><<<grid, 128, 0, s>>>(jobs);
+    count_launch();
+    return cudaGetLastError();
 }
 
 cudaError_t launch_thermal_update_fill(const ThermalArgs& a, int storage, void* f, const IpArgs& fill, cudaStream_t s) {
