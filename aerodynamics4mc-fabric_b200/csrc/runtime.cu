@@ -491,6 +491,7 @@ bool Context::allocate(int nx_, int ny_, int nz_) {
     force_valid = false;
     slot = 0;
     slots_match = false;
+    streamed = false;
     cur = 0;
     step_counter = 0;
     return true;
@@ -984,6 +985,7 @@ static bool step_context_body(Context& ctx, const float* packet, float* out, flo
                 a.transport = 1;
                 a.tr = transport;
             }
+            if (g_streamed_step) ctx.streamed = true;
             if (!cuda_ok(ip_step(ctx.ip_variant, ctx.ip, a, transitions, s), "step_inplace")) return false;
             ctx.parity ^= 1;
         }
@@ -1180,8 +1182,11 @@ bool read_output_box(Context& ctx, OutBox box, int out_ch, float scale, float* h
                      "cudaMemcpyAsync(temperature)"))
             return false;
     }
+    // only a streamed step can set the fault word; its copy (to pageable
+    // memory, so the call waits for it) cost a small brick's call 10 of 36 us
     int fault = 0;
-    if (!cuda_ok(cudaMemcpyAsync(&fault, ctx.fault, sizeof(int), cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync(fault)")) return false;
+    if (ctx.streamed &&
+        !cuda_ok(cudaMemcpyAsync(&fault, ctx.fault, sizeof(int), cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync(fault)")) return false;
     if (!cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize(output)")) return false;
     if (fault) {
         set_error("in-place step: a tile's bulk copies did not complete within the wait limit; the state is invalid");

@@ -49,6 +49,7 @@ struct Context {
     size_t out_cap = 0;
     float* force = nullptr;  // optional per-cell force density, SoA (3 * cells)
     int* fault = nullptr;    // device word: a streamed in-place step lost a tile's copies
+    bool streamed = false;   // a call ran with the streamed step on (the word may have been set)
     FaceParams face_prev{};
     FaceParams h_face[2]{};  // host copies (source of the async uploads; must outlive them)
     // Layout chosen at the first step: 0 two-buffer pull (g[0], g[1]),
