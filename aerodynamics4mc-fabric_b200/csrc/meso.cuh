@@ -46,6 +46,19 @@ struct HydroRates {
     float tau_h, omega_even, omega_odd, smagorinsky_c, fx, fy, fz;
 };
 
+// What the model reads of a call's forcing, per cell, SoA (entry k of cell i
+// at k * cells + i): the 25 channels are one 100-byte record per cell, so a
+// warp's load of one channel touches 25 lines, and the pull read the solid
+// channel of 19 neighbours that way. Derived once per call (meso_launch_derive).
+enum MesoDerived : int {
+    kDLatticeX = 0, kDLatticeY, kDLatticeZ,  // clamped inflow velocity (lattice units)
+    kDSlopeX, kDSlopeZ,                      // terrain slope
+    kDDrag, kDHumidity,
+    kDAmbient, kDDeep, kDSurface,            // target temperatures (the surface one is also the wall's)
+    kDConvHeat, kDTornadoHeat, kDTornadoUp, kDNestedUp,
+    kDCount
+};
+
 // One step of the reference model (hydrodynamic + thermal distributions).
 // Populations are SoA: f[q*cells+cell].
 struct MesoArgs {
@@ -54,12 +67,15 @@ struct MesoArgs {
     float dt_s, velocity_scale, max_speed;
     HydroRates h;
     float omega_t_even, omega_t_odd;
-    const float* forcing;  // cells x 25 (AoS, as passed by the caller)
-    float* f;              // current hydrodynamic populations (19 x cells)
-    float* g;              // current thermal populations (19 x cells)
-    float* post_f;         // post-collision scratch (19 x cells)
-    float* post_g;
-    float* ambient;        // macro temperature of the previous step (read), this step (written)
+    const float* forcing;  // cells x 25 (AoS, as passed by the caller): seed and derivation only
+    float* derived;        // kDCount x cells
+    uint8_t* solid;
+    const uint32_t* flags; // pull classification (meso_hydro_flags)
+    const float* src_f;    // streamed, or (fused step, stream, ambient) post-collision populations
+    const float* src_g;
+    float* dst_f;
+    float* dst_g;
+    float* ambient;        // macro temperature of the streamed state
     float* deep;           // deep-ground / surface temperatures of the previous step
     float* surface;
     float* next_deep;      // ... of this step
@@ -87,7 +103,16 @@ struct HydroArgs {
 }  // namespace meso
 
 cudaError_t meso_launch_seed(const meso::MesoArgs& a, cudaStream_t s);
-cudaError_t meso_launch_step(const meso::MesoArgs& a, cudaStream_t s);
+// Derived forcing and solid mask of a call's forcing.
+cudaError_t meso_launch_derive(const meso::MesoArgs& a, cudaStream_t s);
+// Targets + TRT of the streamed state src into post-collision dst; pull: src
+// holds the last step's post-collision populations, streamed on the way in.
+cudaError_t meso_launch_collide(const meso::MesoArgs& a, bool pull, cudaStream_t s);
+// Temperature (zeroth moment of the streamed thermal populations) of
+// post-collision src: what the neighbours of a fused step's cells read.
+cudaError_t meso_launch_ambient(const meso::MesoArgs& a, cudaStream_t s);
+// Stream post-collision src into dst, macro export.
+cudaError_t meso_launch_stream(const meso::MesoArgs& a, cudaStream_t s);
 
 // Hydrodynamic-only step. `fp16` selects __half deviation storage.
 enum MesoHydroMode { kHydroInit = 0, kHydroStep = 1, kHydroOutput = 2 };
@@ -96,7 +121,8 @@ enum MesoStorage { kMesoStoreF32 = 0, kMesoStoreF16 = 1, kMesoStoreI16 = 2 };
 cudaError_t meso_hydro_seed(const float* forcing, int nx, int ny, int nz, float velocity_scale, int storage, float scale,
                             void* dst, uint8_t* solid, cudaStream_t s);
 cudaError_t meso_hydro_mask(const float* forcing, long long cells, uint8_t* solid, cudaStream_t s);
-// Pull classification word per cell: bit q (0..18) = direction q bounces back,
+// Pull classification word per cell: bit q (0..18) = direction q bounces back
+// (also off a solid cell it would reflect from at the free-slip lid),
 // kHydroSlow = the cell pulls through an open side or the lid, or is blended,
 // kHydroSelfSolid = the cell is solid.
 constexpr uint32_t kHydroSelfSolid = 1u << 31;

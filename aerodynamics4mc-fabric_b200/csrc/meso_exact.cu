@@ -4,15 +4,17 @@
 // and the ground, equilibrium inflow with a two-cell blend at the sides and
 // top, macro export (native/src/aero_lbm_mesoscale.cpp:146-738).
 //
-// Two launches per step: `meso_collide_kernel` (targets + TRT, one thread per
-// cell; writes post-collision f and g and the next surface / deep-ground
-// temperatures) and `meso_stream_kernel` (pull + boundaries + macro export
-// for the cell; writes the new f and g, the ambient field and the output
+// A call from the host is two launches: `meso_collide_kernel` (targets + TRT,
+// one thread per cell; writes post-collision f and g and the next surface /
+// deep-ground temperatures) and `meso_stream_kernel` (pull + boundaries +
+// macro export; writes the new f and g, the ambient field and the output
 // state). The collision needs the neighbours' previous temperatures
 // (laplacians) and the pull needs the neighbours' post-collision populations,
-// so the step has two grid-wide dependencies and cannot be one launch.
-// Populations are structure-of-arrays f[q][cell] (the reference stores
-// f[cell*19+q]; the layout is internal to both).
+// so the step has two grid-wide dependencies and cannot be one launch. Within
+// a window of resident steps the pull moves into the next collision, and the
+// pass between two collisions (`meso_ambient_kernel`) forms the streamed
+// temperature alone. Populations are structure-of-arrays f[q][cell] (the
+// reference stores f[cell*19+q]; the layout is internal to both).
 //
 // This file is built with --fmad=false and every expression keeps the
 // reference's operation order (products by the integer lattice components
@@ -78,19 +80,64 @@ __device__ __forceinline__ float vlap(const MesoArgs& A, const float* __restrict
     return yp + ym - 2.0f * c;
 }
 
+__device__ __forceinline__ float dv(const MesoArgs& A, int k, long long i) {
+    return __ldg(A.derived + k * ((long long)A.nx * A.ny * A.nz) + i);
+}
+
+// The forcing terms of compute_cell_targets and of the open boundaries that
+// do not depend on the state (native/src/aero_lbm_mesoscale.cpp:393-530,
+// 620-734), each expression as the reference has it.
+__global__ void __launch_bounds__(128) meso_derive_kernel(MesoArgs A) {
+    const long long cells = (long long)A.nx * A.ny * A.nz;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= cells) return;
+    int x, y, z;
+    cell_xyz32(i, A.ny, A.nz, x, y, z);
+    const float* F = A.forcing;
+    const float conv_m = ch(F, i, kChConvectiveMoistening), tor_m = ch(F, i, kChTornadoMoistening);
+    const float conv_x = ch(F, i, kChConvectiveInflowX), conv_z = ch(F, i, kChConvectiveInflowZ);
+    const float tor_x = ch(F, i, kChTornadoWindX), tor_z = ch(F, i, kChTornadoWindZ);
+    const float tor_up = ch(F, i, kChTornadoUpdraft), nest_up = ch(F, i, kChNestedUpdraft);
+    const float bx = ch(F, i, kChBackgroundWindX) + ch(F, i, kChNestedWindXDelta) + conv_x + tor_x;
+    const float bz = ch(F, i, kChBackgroundWindZ) + ch(F, i, kChNestedWindZDelta) + conv_z + tor_z;
+    const float by = nest_up + tor_up;
+    const float den = smax(1.0e-6f, A.velocity_scale);
+    const int xp = min(A.nx - 1, x + 1), xm = max(0, x - 1), zp = min(A.nz - 1, z + 1), zm = max(0, z - 1);
+    float v[kDCount];
+    v[kDLatticeX] = clamp_speed(bx / den);
+    v[kDLatticeY] = clamp_speed(by / den);
+    v[kDLatticeZ] = clamp_speed(bz / den);
+    v[kDSlopeX] = 0.5f * (ch(F, midx(A, xp, y, z), kChTerrainHeight) - ch(F, midx(A, xm, y, z), kChTerrainHeight));
+    v[kDSlopeZ] = 0.5f * (ch(F, midx(A, x, y, zp), kChTerrainHeight) - ch(F, midx(A, x, y, zm), kChTerrainHeight));
+    const float rough = smax(0.0f, ch(F, i, kChRoughness));
+    v[kDDrag] = sclamp(rough * 0.02f, 0.0f, 0.25f);
+    v[kDHumidity] = sclamp(ch(F, i, kChHumidity) + conv_m + tor_m, 0.0f, 1.0f);
+    v[kDAmbient] = ch(F, i, kChAmbientTarget) + ch(F, i, kChNestedAmbientDelta);
+    v[kDDeep] = ch(F, i, kChDeepGroundTarget);
+    v[kDSurface] = wall_temp(F, i);
+    v[kDConvHeat] = ch(F, i, kChConvectiveHeating);
+    v[kDTornadoHeat] = ch(F, i, kChTornadoHeating);
+    v[kDTornadoUp] = tor_up;
+    v[kDNestedUp] = nest_up;
+    A.solid[i] = solid_at(F, i) ? 1 : 0;
+#pragma unroll
+    for (int k = 0; k < kDCount; ++k) A.derived[k * cells + i] = v[k];
+}
+
 struct Targets {
     float rho, ux, uy, uz, teq, nsurf, ndeep;
 };
 
 // compute_cell_targets (native/src/aero_lbm_mesoscale.cpp:393-530)
 __device__ __forceinline__ Targets cell_targets(const MesoArgs& A, const float (&f)[19], const float (&g)[19], long long i,
-                                                int x, int y, int z) {
-    const float* F = A.forcing;
+                                                int x, int y, int z, bool solid) {
     const float dt = smax(1.0e-3f, A.dt_s);
     const float amb_relax = sclamp(dt / 600.0f, 0.0f, 1.0f);
     const float deep_relax = sclamp(dt / 2400.0f, 0.0f, 1.0f);
     const float surf_relax = sclamp(dt / 300.0f, 0.0f, 1.0f);
     const float wind_relax = sclamp(dt / 60.0f, 0.0f, 1.0f);
+    const float deep_t = dv(A, kDDeep, i), surf_t = dv(A, kDSurface, i);
+    if (solid) return Targets{1.0f, 0.0f, 0.0f, 0.0f, surf_t, surf_t, deep_t};
     float r = 0.0f, ux = 0.0f, uy = 0.0f, uz = 0.0f, amb = 0.0f;
 #pragma unroll
     for (int q = 0; q < 19; ++q) {
@@ -104,24 +151,11 @@ __device__ __forceinline__ Targets cell_targets(const MesoArgs& A, const float (
     ux /= r;
     uy /= r;
     uz /= r;
-    const float amb_t = ch(F, i, kChAmbientTarget) + ch(F, i, kChNestedAmbientDelta);
-    const float deep_t = ch(F, i, kChDeepGroundTarget);
-    const float surf_t = ch(F, i, kChSurfaceTarget) + ch(F, i, kChNestedSurfaceDelta);
-    if (solid_at(F, i)) return Targets{1.0f, 0.0f, 0.0f, 0.0f, surf_t, surf_t, deep_t};
-    const float rough = smax(0.0f, ch(F, i, kChRoughness));
-    const float conv_h = ch(F, i, kChConvectiveHeating), conv_m = ch(F, i, kChConvectiveMoistening);
-    const float conv_x = ch(F, i, kChConvectiveInflowX), conv_z = ch(F, i, kChConvectiveInflowZ);
-    const float tor_x = ch(F, i, kChTornadoWindX), tor_z = ch(F, i, kChTornadoWindZ);
-    const float tor_h = ch(F, i, kChTornadoHeating), tor_m = ch(F, i, kChTornadoMoistening);
-    const float tor_up = ch(F, i, kChTornadoUpdraft), nest_up = ch(F, i, kChNestedUpdraft);
-    const float nest_dx = ch(F, i, kChNestedWindXDelta), nest_dz = ch(F, i, kChNestedWindZDelta);
-    const float bx = ch(F, i, kChBackgroundWindX) + nest_dx + conv_x + tor_x;
-    const float bz = ch(F, i, kChBackgroundWindZ) + nest_dz + conv_z + tor_z;
-    const float by = nest_up + tor_up;
-    const float hum = sclamp(ch(F, i, kChHumidity) + conv_m + tor_m, 0.0f, 1.0f);
-    const int xp = min(A.nx - 1, x + 1), xm = max(0, x - 1), zp = min(A.nz - 1, z + 1), zm = max(0, z - 1);
-    const float sx = 0.5f * (ch(F, midx(A, xp, y, z), kChTerrainHeight) - ch(F, midx(A, xm, y, z), kChTerrainHeight));
-    const float sz = 0.5f * (ch(F, midx(A, x, y, zp), kChTerrainHeight) - ch(F, midx(A, x, y, zm), kChTerrainHeight));
+    const float amb_t = dv(A, kDAmbient, i);
+    const float conv_h = dv(A, kDConvHeat, i), tor_h = dv(A, kDTornadoHeat, i);
+    const float tor_up = dv(A, kDTornadoUp, i), nest_up = dv(A, kDNestedUp, i);
+    const float hum = dv(A, kDHumidity, i);
+    const float sx = dv(A, kDSlopeX, i), sz = dv(A, kDSlopeZ, i);
     const float s_hl = hlap(A, A.surface, x, y, z), s_vl = vlap(A, A.surface, x, y, z);
     const float d_vl = vlap(A, A.deep, x, y, z);
     const float a_hl = hlap(A, A.ambient, x, y, z), a_vl = vlap(A, A.ambient, x, y, z);
@@ -130,15 +164,14 @@ __device__ __forceinline__ Targets cell_targets(const MesoArgs& A, const float (
     const float damp = 1.0f - 0.12f * hum;
     const float nsurf = surf_i + surf_relax * damp * (surf_t - surf_i) + 0.10f * (ndeep - surf_i) + 0.04f * conv_h +
                         0.08f * tor_h + 0.05f * s_hl + 0.025f * s_vl;
-    const float den = smax(1.0e-6f, A.velocity_scale);
-    const float lx = clamp_speed(bx / den), ly = clamp_speed(by / den), lz = clamp_speed(bz / den);
+    const float lx = dv(A, kDLatticeX, i), ly = dv(A, kDLatticeY, i), lz = dv(A, kDLatticeZ, i);
     const float push = 0.0008f * (nsurf - amb);
     const float nsw = 1.0f - (float)y / smax(1.0f, (float)(A.ny - 1));
     const float lift = 0.0015f * (lx * sx + lz * sz) * nsw;
     const float blift = 0.0009f * (nsurf - amb) * nsw;
     const float steer_x = -0.005f * sx * lz;
     const float steer_z = 0.005f * sz * lx;
-    const float drag = sclamp(rough * 0.02f, 0.0f, 0.25f);
+    const float drag = dv(A, kDDrag, i);
     const float tux = clamp_speed(lx + steer_x + push * sx - drag * ux);
     const float tuz = clamp_speed(lz + steer_z + push * sz - drag * uz);
     const float tuy = clamp_speed(ly + lift + blift - drag * uy);
@@ -211,81 +244,69 @@ __device__ __forceinline__ void trt_hydro(const HydroRates& H, const float (&f)[
     }
 }
 
-// Targets + TRT of both distributions (native/src/aero_lbm_mesoscale.cpp:573-618).
-__global__ void __launch_bounds__(128) meso_collide_kernel(MesoArgs A) {
-    const long long cells = (long long)A.nx * A.ny * A.nz;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cells) return;
-    int x, y, z;
-    cell_xyz32(i, A.ny, A.nz, x, y, z);
-    float f[19], g[19];
-#pragma unroll
-    for (int q = 0; q < 19; ++q) {
-        f[q] = A.f[q * cells + i];
-        g[q] = A.g[q * cells + i];
-    }
-    const Targets t = cell_targets(A, f, g, i, x, y, z);
-    A.next_deep[i] = t.ndeep;
-    A.next_surface[i] = t.nsurf;
-    float pf[19];
-    trt_hydro(A.h, f, t.rho, t.ux, t.uy, t.uz, solid_at(A.forcing, i), pf);
-    const float om_t_even = A.omega_t_even, om_t_odd = A.omega_t_odd;
-#pragma unroll
-    for (int q = 0; q < 19; ++q) {
-        A.post_f[q * cells + i] = pf[q];
-        const int qo = mopp(q);
-        if (q > qo) continue;
-        if (q == qo) {
-            const float ge = tfeq(q, t.teq, t.ux, t.uy, t.uz);
-            A.post_g[q * cells + i] = g[q] - om_t_even * (g[q] - ge);
-            continue;
-        }
-        const float ge = tfeq(q, t.teq, t.ux, t.uy, t.uz), geo = tfeq(qo, t.teq, t.ux, t.uy, t.uz);
-        const float gev = 0.5f * (g[q] + g[qo]), god = 0.5f * (g[q] - g[qo]);
-        const float geev = 0.5f * (ge + geo), geod = 0.5f * (ge - geo);
-        const float gep = gev - om_t_even * (gev - geev);
-        const float gop = god - om_t_odd * (god - geod);
-        A.post_g[q * cells + i] = gep + gop;
-        A.post_g[qo * cells + i] = gep - gop;
-    }
+// Directions whose component along an axis is +1 / -1, as a bit set.
+__host__ __device__ constexpr uint32_t mdirs(int axis, int sign) {
+    uint32_t m = 0;
+    for (int q = 0; q < 19; ++q)
+        if ((axis == 0 ? mcx(q) : (axis == 1 ? mcy(q) : mcz(q))) == sign) m |= 1u << q;
+    return m;
 }
 
-// Pull streaming, boundaries and macro export
-// (native/src/aero_lbm_mesoscale.cpp:620-734).
-__global__ void __launch_bounds__(128) meso_stream_kernel(MesoArgs A) {
+// Streamed populations of cell i from the post-collision ones (pull
+// streaming, native/src/aero_lbm_mesoscale.cpp:620-734). Every population is
+// one load at an address formed by selects, the same for interior and
+// boundary cells (half of the warps hold cells of an open side: as separate
+// paths each of their 38 loads waited twice); cells that pull through an open
+// side or the lid, or are blended, then replace or blend the values.
+// kHydro false: the thermal populations only. I: unsigned where 19 x cells
+// fits 32 bits.
+template <bool kHydro, class I>
+__device__ __forceinline__ void pull_model(const MesoArgs& A, long long i, int x, int y, int z, uint32_t w, float (&fn)[19],
+                                           float (&gn)[19]) {
     const int nx = A.nx, ny = A.ny, nz = A.nz;
-    const long long cells = (long long)nx * ny * nz;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cells) return;
-    int x, y, z;
-    cell_xyz32(i, ny, nz, x, y, z);
-    const float* F = A.forcing;
-    float* out = A.out_state ? A.out_state + i * kMesoStateChannels : nullptr;
-    if (solid_at(F, i)) {
-        const float wt = wall_temp(F, i);
+    const I cells = (I)nx * (I)ny * (I)nz, own = (I)i;
+    const float* __restrict__ pf = A.src_f;
+    const float* __restrict__ pg = A.src_g;
+    const float* __restrict__ wall = A.derived + kDSurface * (long long)cells;
+    if (w & kHydroSelfSolid) {
+        const float wt = __ldg(wall + i);
 #pragma unroll
         for (int q = 0; q < 19; ++q) {
-            A.f[q * cells + i] = hfeq(q, 1.0f, 0.0f, 0.0f, 0.0f);
-            A.g[q * cells + i] = tfeq(q, wt, 0.0f, 0.0f, 0.0f);
-        }
-        A.ambient[i] = wt;
-        if (out) {
-            out[0] = wt;
-            out[1] = A.next_deep[i];
-            out[2] = A.next_surface[i];
-            out[3] = 0.0f;
-            out[4] = 0.0f;
-            out[5] = 0.0f;
+            if (kHydro) fn[q] = hfeq(q, 1.0f, 0.0f, 0.0f, 0.0f);
+            gn[q] = tfeq(q, wt, 0.0f, 0.0f, 0.0f);
         }
         return;
     }
-    const float den = smax(1.0e-6f, A.velocity_scale);
-    const float bx = clamp_speed((ch(F, i, kChBackgroundWindX) + ch(F, i, kChNestedWindXDelta) + ch(F, i, kChConvectiveInflowX) +
-                                  ch(F, i, kChTornadoWindX)) / den);
-    const float bz = clamp_speed((ch(F, i, kChBackgroundWindZ) + ch(F, i, kChNestedWindZDelta) + ch(F, i, kChConvectiveInflowZ) +
-                                  ch(F, i, kChTornadoWindZ)) / den);
-    const float btemp = ch(F, i, kChAmbientTarget) + ch(F, i, kChNestedAmbientDelta);
-    const float by = clamp_speed((ch(F, i, kChNestedUpdraft) + ch(F, i, kChTornadoUpdraft)) / den);
+    // neighbour terms per axis: wrapped sides (a pull through an open side
+    // loads an unused value there), the grid's own row at the ground and the lid
+    I X[3], Y[3], Z[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int sx = x + k - 1, sy = y + k - 1, sz = z + k - 1;
+        X[k] = (I)(sx < 0 ? sx + nx : (sx >= nx ? sx - nx : sx)) * ((I)ny * (I)nz);
+        Y[k] = (I)min(max(sy, 0), ny - 1) * (I)nz;
+        Z[k] = (I)(sz < 0 ? sz + nz : (sz >= nz ? sz - nz : sz));
+    }
+    const uint32_t ground = y == 0 ? mdirs(1, 1) : 0u, lid = (A.free_slip_top && y == ny - 1) ? mdirs(1, -1) : 0u;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) {
+        const bool bounced = (w >> q) & 1u;
+        const I src = ((ground >> q) & 1u) ? own : X[1 - mcx(q)] + Y[1 - mcy(q)] + Z[1 - mcz(q)];
+        // specular reflection at the lid: the mirrored population of the same row
+        const I from = (mcy(q) == -1 && (lid >> q) & 1u) ? (I)mmirror(q) * cells + src : (I)q * cells + src;
+        if (kHydro) fn[q] = __ldg(pf + (bounced ? (I)mopp(q) * cells + own : from));
+        gn[q] = __ldg(bounced ? wall + src : pg + from);
+    }
+#pragma unroll
+    for (int q = 0; q < 19; ++q)
+        if ((w >> q) & 1u) gn[q] = tfeq(q, gn[q], 0.0f, 0.0f, 0.0f);
+    if (!(w & kHydroSlow)) return;
+    uint32_t away = 0;
+    if (!A.periodic_sides)
+        away = (x == 0 ? mdirs(0, 1) : 0u) | (x == nx - 1 ? mdirs(0, -1) : 0u) | (z == 0 ? mdirs(2, 1) : 0u) |
+               (z == nz - 1 ? mdirs(2, -1) : 0u);
+    if (!A.free_slip_top && y == ny - 1) away |= mdirs(1, -1);
+    away &= ~ground;
     int edge = min(min(x, z), min(nx - 1 - x, nz - 1 - z));
     int top = ny - 1 - y;
     if (A.periodic_sides) edge = 1 << 20;
@@ -293,58 +314,124 @@ __global__ void __launch_bounds__(128) meso_stream_kernel(MesoArgs A) {
     const int sponge = min(edge, top);
     float alpha = sponge <= 0 ? 1.0f : (sponge < 2 ? 0.5f : 0.0f);
     if (!A.edge_blend) alpha = 0.0f;
-    float fn[19], gn[19];
+    const float bx = dv(A, kDLatticeX, i), by = dv(A, kDLatticeY, i), bz = dv(A, kDLatticeZ, i), btemp = dv(A, kDAmbient, i);
 #pragma unroll
     for (int q = 0; q < 19; ++q) {
-        int sx = x - mcx(q), sy = y - mcy(q), sz = z - mcz(q);
-        if (A.periodic_sides) {
-            sx = (sx + nx) % nx;
-            sz = (sz + nz) % nz;
+        if (((w >> q) & 1u) && !((away >> q) & 1u)) continue;
+        const float fb = kHydro ? hfeq(q, 1.0f, bx, by, bz) : 0.0f, gb = tfeq(q, btemp, bx, by, bz);
+        if ((away >> q) & 1u) {
+            if (kHydro) fn[q] = fb;
+            gn[q] = gb;
         }
-        float fv, gv;
-        bool bounced = false;
-        if (sx >= 0 && sx < nx && sy >= 0 && sy < ny && sz >= 0 && sz < nz) {
-            const long long src = midx(A, sx, sy, sz);
-            if (solid_at(F, src)) {
-                fv = A.post_f[mopp(q) * cells + i];
-                gv = tfeq(q, wall_temp(F, src), 0.0f, 0.0f, 0.0f);
-                bounced = true;
-            } else {
-                fv = A.post_f[q * cells + src];
-                gv = A.post_g[q * cells + src];
-            }
-        } else if (sy < 0) {
-            fv = A.post_f[mopp(q) * cells + i];
-            gv = tfeq(q, wall_temp(F, i), 0.0f, 0.0f, 0.0f);
-            bounced = true;
-        } else if (A.free_slip_top && sy >= ny && sx >= 0 && sx < nx && sz >= 0 && sz < nz) {
-            const long long src = midx(A, sx, ny - 1, sz);
-            if (solid_at(F, src)) {
-                fv = A.post_f[mopp(q) * cells + i];
-                gv = tfeq(q, wall_temp(F, src), 0.0f, 0.0f, 0.0f);
-                bounced = true;
-            } else {
-                fv = A.post_f[mmirror(q) * cells + src];
-                gv = A.post_g[mmirror(q) * cells + src];
-            }
-        } else {
-            fv = hfeq(q, 1.0f, bx, by, bz);
-            gv = tfeq(q, btemp, bx, by, bz);
+        if (alpha > 0.0f) {
+            if (kHydro) fn[q] = (1.0f - alpha) * fn[q] + alpha * fb;
+            gn[q] = (1.0f - alpha) * gn[q] + alpha * gb;
         }
-        if (alpha > 0.0f && !bounced) {
-            const float fb = hfeq(q, 1.0f, bx, by, bz);
-            const float gb = tfeq(q, btemp, bx, by, bz);
-            fv = (1.0f - alpha) * fv + alpha * fb;
-            gv = (1.0f - alpha) * gv + alpha * gb;
+    }
+}
+
+// Targets + TRT of both distributions (native/src/aero_lbm_mesoscale.cpp:573-618).
+// kPull: the last step's streaming on the way in, so that a window of steps
+// reads and writes the populations once per step instead of twice
+// (128 x 24 x 128: 63 us a step with the ambient pass, 110 as collide +
+// stream over the forcing records).
+template <bool kPull, class I>
+__global__ void __launch_bounds__(128) meso_collide_kernel(MesoArgs A) {
+    const long long cells = (long long)A.nx * A.ny * A.nz;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= cells) return;
+    int x, y, z;
+    cell_xyz32(i, A.ny, A.nz, x, y, z);
+    const uint32_t w = A.flags[i];
+    float f[19], g[19];
+    if (kPull) {
+        pull_model<true, I>(A, i, x, y, z, w, f, g);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 19; ++q) {
+            f[q] = A.src_f[q * cells + i];
+            g[q] = A.src_g[q * cells + i];
         }
-        fn[q] = fv;
-        gn[q] = gv;
+    }
+    const bool solid = (w & kHydroSelfSolid) != 0;
+    const Targets t = cell_targets(A, f, g, i, x, y, z, solid);
+    A.next_deep[i] = t.ndeep;
+    A.next_surface[i] = t.nsurf;
+    float pf[19];
+    trt_hydro(A.h, f, t.rho, t.ux, t.uy, t.uz, solid, pf);
+    const float om_t_even = A.omega_t_even, om_t_odd = A.omega_t_odd;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) {
+        A.dst_f[q * cells + i] = pf[q];
+        const int qo = mopp(q);
+        if (q > qo) continue;
+        if (q == qo) {
+            const float ge = tfeq(q, t.teq, t.ux, t.uy, t.uz);
+            A.dst_g[q * cells + i] = g[q] - om_t_even * (g[q] - ge);
+            continue;
+        }
+        const float ge = tfeq(q, t.teq, t.ux, t.uy, t.uz), geo = tfeq(qo, t.teq, t.ux, t.uy, t.uz);
+        const float gev = 0.5f * (g[q] + g[qo]), god = 0.5f * (g[q] - g[qo]);
+        const float geev = 0.5f * (ge + geo), geod = 0.5f * (ge - geo);
+        const float gep = gev - om_t_even * (gev - geev);
+        const float gop = god - om_t_odd * (god - geod);
+        A.dst_g[q * cells + i] = gep + gop;
+        A.dst_g[qo * cells + i] = gep - gop;
+    }
+}
+
+template <class I>
+__global__ void __launch_bounds__(128) meso_ambient_kernel(MesoArgs A) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)A.nx * A.ny * A.nz) return;
+    int x, y, z;
+    cell_xyz32(i, A.ny, A.nz, x, y, z);
+    const uint32_t w = A.flags[i];
+    if (w & kHydroSelfSolid) {
+        A.ambient[i] = dv(A, kDSurface, i);
+        return;
+    }
+    float f[19], g[19];
+    pull_model<false, I>(A, i, x, y, z, w, f, g);
+    float amb = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) amb += g[q];
+    A.ambient[i] = amb;
+}
+
+// Pull streaming and macro export (native/src/aero_lbm_mesoscale.cpp:620-734).
+template <class I>
+__global__ void __launch_bounds__(128) meso_stream_kernel(MesoArgs A) {
+    const long long cells = (long long)A.nx * A.ny * A.nz;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= cells) return;
+    int x, y, z;
+    cell_xyz32(i, A.ny, A.nz, x, y, z);
+    const uint32_t w = A.flags[i];
+    float* out = A.out_state ? A.out_state + i * kMesoStateChannels : nullptr;
+    float fn[19], gn[19];
+    pull_model<true, I>(A, i, x, y, z, w, fn, gn);
+#pragma unroll
+    for (int q = 0; q < 19; ++q) {
+        A.dst_f[q * cells + i] = fn[q];
+        A.dst_g[q * cells + i] = gn[q];
+    }
+    if (w & kHydroSelfSolid) {
+        const float wt = dv(A, kDSurface, i);
+        A.ambient[i] = wt;
+        if (out) {
+            out[0] = wt;
+            out[1] = A.deep[i];
+            out[2] = A.surface[i];
+            out[3] = 0.0f;
+            out[4] = 0.0f;
+            out[5] = 0.0f;
+        }
+        return;
     }
     float r = 0.0f, ux = 0.0f, uy = 0.0f, uz = 0.0f, amb = 0.0f;
 #pragma unroll
     for (int q = 0; q < 19; ++q) {
-        A.f[q * cells + i] = fn[q];
-        A.g[q * cells + i] = gn[q];
         r += fn[q];
         ux += fn[q] * fx_(q);
         uy += fn[q] * fy_(q);
@@ -359,8 +446,8 @@ __global__ void __launch_bounds__(128) meso_stream_kernel(MesoArgs A) {
     if (out) {
         const float ms = A.max_speed;
         out[0] = amb;
-        out[1] = A.next_deep[i];
-        out[2] = A.next_surface[i];
+        out[1] = A.deep[i];
+        out[2] = A.surface[i];
         out[3] = sclamp(ux * A.velocity_scale, -ms, ms);
         out[4] = sclamp(uy * A.velocity_scale, -ms, ms);
         out[5] = sclamp(uz * A.velocity_scale, -ms, ms);
@@ -389,8 +476,8 @@ __global__ void meso_seed_kernel(MesoArgs A) {
     A.surface[i] = surf_t;
 #pragma unroll
     for (int q = 0; q < 19; ++q) {
-        A.f[q * cells + i] = hfeq(q, 1.0f, lx, ly, lz);
-        A.g[q * cells + i] = tfeq(q, amb, lx, ly, lz);
+        A.dst_f[q * cells + i] = hfeq(q, 1.0f, lx, ly, lz);
+        A.dst_g[q * cells + i] = tfeq(q, amb, lx, ly, lz);
     }
 }
 
@@ -568,7 +655,10 @@ __global__ void meso_hydro_seed_kernel(const float* __restrict__ F, int nx, int 
     for (int q = 0; q < 19; ++q) S::store(dst + q * cells + i, q, hfeq(q, 1.0f, lx, ly, lz), scale);
 }
 
-// Pull classification of a mask (see meso_hydro_flags).
+// Pull classification of a mask (see meso_hydro_flags): the 19 mask bytes are
+// loaded whatever the cell's place (an open side's from the wrapped cell, the
+// ground's and the lid's from the cell's own row), so they do not wait for
+// one another.
 __global__ void meso_hydro_flags_kernel(HydroArgs A, const uint8_t* __restrict__ solid, uint32_t* __restrict__ flags) {
     const int nx = A.nx, ny = A.ny, nz = A.nz;
     const long long cells = (long long)nx * ny * nz;
@@ -580,27 +670,32 @@ __global__ void meso_hydro_flags_kernel(HydroArgs A, const uint8_t* __restrict__
     }
     int x, y, z;
     cell_xyz32(i, ny, nz, x, y, z);
+    long long X[3], Y[3], Z[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int sx = x + k - 1, sy = y + k - 1, sz = z + k - 1;
+        X[k] = (long long)(sx < 0 ? sx + nx : (sx >= nx ? sx - nx : sx)) * ny * nz;
+        Y[k] = (long long)min(max(sy, 0), ny - 1) * nz;
+        Z[k] = sz < 0 ? sz + nz : (sz >= nz ? sz - nz : sz);
+    }
+    uint32_t hit = 0;
+#pragma unroll
+    for (int q = 0; q < 19; ++q)
+        hit |= __ldg(solid + X[1 - mcx(q)] + Y[1 - mcy(q)] + Z[1 - mcz(q)]) ? 1u << q : 0u;
+    uint32_t side = 0;
+    if (!A.periodic_sides)
+        side = (x == 0 ? mdirs(0, 1) : 0u) | (x == nx - 1 ? mdirs(0, -1) : 0u) | (z == 0 ? mdirs(2, 1) : 0u) |
+               (z == nz - 1 ? mdirs(2, -1) : 0u);
+    const uint32_t ground = y == 0 ? mdirs(1, 1) : 0u, lid = y == ny - 1 ? mdirs(1, -1) : 0u;
+    // inside the grid (or reflected at a free-slip lid): off the solid cell
+    // there; the ground always; an open side or lid never
+    const uint32_t open = (side | (A.free_slip_top ? 0u : lid)) & ~ground;
+    const uint32_t w = (hit & ~open) | ground;
     int edge = min(min(x, z), min(nx - 1 - x, nz - 1 - z));
     int top = ny - 1 - y;
     if (A.periodic_sides) edge = 1 << 20;
     if (A.free_slip_top) top = 1 << 20;
-    const int sponge = min(edge, top);
-    bool slow = A.edge_blend && sponge < 2;
-    uint32_t w = 0;
-    for (int q = 0; q < 19; ++q) {
-        int sx = x - mcx(q), sy = y - mcy(q), sz = z - mcz(q);
-        if (A.periodic_sides) {
-            sx = sx < 0 ? sx + nx : (sx >= nx ? sx - nx : sx);
-            sz = sz < 0 ? sz + nz : (sz >= nz ? sz - nz : sz);
-        }
-        if (sx >= 0 && sx < nx && sy >= 0 && sy < ny && sz >= 0 && sz < nz) {
-            if (solid[midx(A, sx, sy, sz)]) w |= 1u << q;
-        } else if (sy < 0) {
-            w |= 1u << q;
-        } else {
-            slow = true;
-        }
-    }
+    const bool slow = (A.edge_blend && min(edge, top) < 2) || ((side | lid) & ~ground) != 0;
     flags[i] = w | (slow ? kHydroSlow : 0u);
 }
 
@@ -618,14 +713,36 @@ cudaError_t meso_launch_seed(const meso::MesoArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t meso_launch_step(const meso::MesoArgs& a, cudaStream_t s) {
-    const long long cells = (long long)a.nx * a.ny * a.nz;
-    const unsigned blocks = (unsigned)((cells + 127) / 128);
-    meso::meso_collide_kernel<<<blocks, 128, 0, s>>>(a);
+static unsigned model_blocks(const meso::MesoArgs& a) { return (unsigned)(((long long)a.nx * a.ny * a.nz + 127) / 128); }
+
+cudaError_t meso_launch_derive(const meso::MesoArgs& a, cudaStream_t s) {
+    meso::meso_derive_kernel<<<model_blocks(a), 128, 0, s>>>(a);
     count_launch();
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    meso::meso_stream_kernel<<<blocks, 128, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+// 32-bit population indices where they fit.
+static bool model_narrow(const meso::MesoArgs& a) { return 19LL * a.nx * a.ny * a.nz < (1LL << 32); }
+
+cudaError_t meso_launch_collide(const meso::MesoArgs& a, bool pull, cudaStream_t s) {
+    using Wide = unsigned long long;
+    if (!pull) meso::meso_collide_kernel<false, Wide><<<model_blocks(a), 128, 0, s>>>(a);
+    else if (model_narrow(a)) meso::meso_collide_kernel<true, unsigned><<<model_blocks(a), 128, 0, s>>>(a);
+    else meso::meso_collide_kernel<true, Wide><<<model_blocks(a), 128, 0, s>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t meso_launch_ambient(const meso::MesoArgs& a, cudaStream_t s) {
+    if (model_narrow(a)) meso::meso_ambient_kernel<unsigned><<<model_blocks(a), 128, 0, s>>>(a);
+    else meso::meso_ambient_kernel<unsigned long long><<<model_blocks(a), 128, 0, s>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t meso_launch_stream(const meso::MesoArgs& a, cudaStream_t s) {
+    if (model_narrow(a)) meso::meso_stream_kernel<unsigned><<<model_blocks(a), 128, 0, s>>>(a);
+    else meso::meso_stream_kernel<unsigned long long><<<model_blocks(a), 128, 0, s>>>(a);
     count_launch();
     return cudaGetLastError();
 }

@@ -70,6 +70,7 @@ struct MesoContext {
     int fslot = 0;          // forcing / mask of the last step call
     // reference model
     float *f = nullptr, *g = nullptr, *pf = nullptr, *pg = nullptr;
+    float* derived = nullptr;  // the forcing terms the model reads (meso::MesoDerived)
     float *ambient = nullptr, *deep = nullptr, *surface = nullptr, *ndeep = nullptr, *nsurf = nullptr;
     // hydrodynamic only
     void* pop[2] = {nullptr, nullptr};
@@ -81,13 +82,13 @@ struct MesoContext {
     void release() {
         for (void* p : {(void*)forcing[0], (void*)forcing[1], (void*)solid[0], (void*)solid[1], (void*)flags[0],
                         (void*)flags[1], (void*)f, (void*)g,
-                        (void*)pf, (void*)pg, (void*)ambient, (void*)deep, (void*)surface, (void*)ndeep, (void*)nsurf,
+                        (void*)pf, (void*)pg, (void*)derived, (void*)ambient, (void*)deep, (void*)surface, (void*)ndeep, (void*)nsurf,
                         pop[0], pop[1], (void*)out})
             if (p) cudaFree(p);
         forcing[0] = forcing[1] = nullptr;
         solid[0] = solid[1] = nullptr;
         flags[0] = flags[1] = nullptr;
-        f = g = pf = pg = ambient = deep = surface = ndeep = nsurf = out = nullptr;
+        f = g = pf = pg = derived = ambient = deep = surface = ndeep = nsurf = out = nullptr;
         pop[0] = pop[1] = nullptr;
         cells = 0;
         initialized = false;
@@ -95,8 +96,8 @@ struct MesoContext {
     }
     double bytes_per_step() const {
         if (hydro) return (double)cells * (19.0 * 2.0 * (storage ? 2.0 : 4.0) + 1.0);
-        // collide: f, g read + written; stream: post f, g read, f, g written; forcing 2 x 100 B; fields; output
-        return (double)cells * (19.0 * 4.0 * 8.0 + 2.0 * 100.0 + 10.0 * 4.0 + 24.0);
+        // fused step: f, g read + written; ambient pass: g read; derived forcing, fields, classification
+        return (double)cells * (19.0 * 4.0 * 5.0 + meso::kDCount * 4.0 + 10.0 * 4.0 + 8.0);
     }
 };
 
@@ -127,7 +128,8 @@ bool allocate(MesoContext& c) {
         ok = cuda_ok(cudaMalloc(&c.pop[0], bytes), "meso populations") && cuda_ok(cudaMalloc(&c.pop[1], bytes), "meso populations") &&
              dev_alloc(&c.flags[0], n, "meso flags") && dev_alloc(&c.flags[1], n, "meso flags");
     } else {
-        ok = dev_alloc(&c.f, n * 19, "meso f") && dev_alloc(&c.g, n * 19, "meso g") && dev_alloc(&c.pf, n * 19, "meso post f") &&
+        ok = dev_alloc(&c.derived, n * meso::kDCount, "meso derived forcing") && dev_alloc(&c.flags[0], n, "meso flags") &&
+             dev_alloc(&c.f, n * 19, "meso f") && dev_alloc(&c.g, n * 19, "meso g") && dev_alloc(&c.pf, n * 19, "meso post f") &&
              dev_alloc(&c.pg, n * 19, "meso post g") && dev_alloc(&c.ambient, n, "meso ambient") &&
              dev_alloc(&c.deep, n, "meso deep") && dev_alloc(&c.surface, n, "meso surface") &&
              dev_alloc(&c.ndeep, n, "meso deep") && dev_alloc(&c.nsurf, n, "meso surface");
@@ -166,10 +168,9 @@ meso::MesoArgs model_args(MesoContext& c, const Transport& t, int slot, float* o
     a.omega_t_even = 1.0f / tau_t;
     a.omega_t_odd = 1.0f / trt_odd_tau(tau_t);
     a.forcing = c.forcing[slot];
-    a.f = c.f;
-    a.g = c.g;
-    a.post_f = c.pf;
-    a.post_g = c.pg;
+    a.derived = c.derived;
+    a.solid = c.solid[0];
+    a.flags = c.flags[0];
     a.ambient = c.ambient;
     a.deep = c.deep;
     a.surface = c.surface;
@@ -204,11 +205,54 @@ meso::HydroArgs hydro_args(const MesoContext& c, const Transport& t, int prev_sl
 
 int hydro_threads(const MesoContext& c) { return c.opt.threads > 0 ? c.opt.threads : 256; }
 
-// One step of the reference model on forcing slot `slot` (two launches).
-bool model_step(MesoContext& c, const Transport& t, int slot, cudaStream_t s) {
-    if (!cuda_ok(meso_launch_step(model_args(c, t, slot, c.out), s), "mesoscale step")) return false;
-    std::swap(c.deep, c.ndeep);
-    std::swap(c.surface, c.nsurf);
+// The derived forcing, mask and pull classification of forcing slot `slot`.
+bool model_inputs(MesoContext& c, const Transport& t, int slot, cudaStream_t s) {
+    meso::HydroArgs h = {};
+    h.nx = c.nx;
+    h.ny = c.ny;
+    h.nz = c.nz;
+    h.periodic_sides = c.opt.periodic_sides ? 1 : 0;
+    h.free_slip_top = c.opt.free_slip_top ? 1 : 0;
+    h.edge_blend = c.opt.disable_edge_blend ? 0 : 1;
+    return cuda_ok(meso_launch_derive(model_args(c, t, slot, nullptr), s), "mesoscale forcing") &&
+           cuda_ok(meso_hydro_flags(h, c.solid[0], c.flags[0], s), "mesoscale flags");
+}
+
+// `steps` steps of the reference model on forcing slot `slot`: collide the
+// streamed state, then for every further step the ambient pass and the fused
+// pull + collision between the two population pairs, then one stream.
+bool model_steps(MesoContext& c, const Transport& t, int slot, int steps, cudaStream_t s) {
+    if (steps < 1) return true;
+    meso::MesoArgs a = model_args(c, t, slot, c.out);
+    auto advance_ground = [&] {
+        std::swap(c.deep, c.ndeep);
+        std::swap(c.surface, c.nsurf);
+        std::swap(a.deep, a.next_deep);
+        std::swap(a.surface, a.next_surface);
+    };
+    a.src_f = c.f;
+    a.src_g = c.g;
+    a.dst_f = c.pf;
+    a.dst_g = c.pg;
+    if (!cuda_ok(meso_launch_collide(a, false, s), "mesoscale step")) return false;
+    advance_ground();
+    for (int k = 1; k < steps; ++k) {
+        // post-collision populations in (pf, pg); the other pair is free
+        a.src_f = c.pf;
+        a.src_g = c.pg;
+        a.dst_f = c.f;
+        a.dst_g = c.g;
+        std::swap(c.f, c.pf);
+        std::swap(c.g, c.pg);
+        if (!cuda_ok(meso_launch_ambient(a, s), "mesoscale ambient") || !cuda_ok(meso_launch_collide(a, true, s), "mesoscale step"))
+            return false;
+        advance_ground();
+    }
+    a.src_f = c.pf;
+    a.src_g = c.pg;
+    a.dst_f = c.f;
+    a.dst_g = c.g;
+    if (!cuda_ok(meso_launch_stream(a, s), "mesoscale stream")) return false;
     c.out_valid = true;
     return true;
 }
@@ -345,12 +389,16 @@ AERO_LBM_B200_EXPORT int aero_lbm_mesoscale_step_context(long long key, const Ae
         c->fslot = slot;
         if (!hydro_output(*c, t, s)) return 0;
     } else {
+        if (!model_inputs(*c, t, slot, s)) return 0;
         if (!c->initialized) {
-            if (!cuda_ok(meso_launch_seed(model_args(*c, t, slot, nullptr), s), "mesoscale seed")) return 0;
+            meso::MesoArgs a = model_args(*c, t, slot, nullptr);
+            a.dst_f = c->f;
+            a.dst_g = c->g;
+            if (!cuda_ok(meso_launch_seed(a, s), "mesoscale seed")) return 0;
             c->initialized = true;
         }
         c->fslot = slot;
-        if (!model_step(*c, t, slot, s)) return 0;
+        if (!model_steps(*c, t, slot, 1, s)) return 0;
     }
     const size_t obytes = (size_t)c->cells * kMesoStateChannels * sizeof(float);
     if (!cuda_ok(cudaMemcpyAsync(out_state, c->out, obytes, cudaMemcpyDeviceToHost, s), "mesoscale output copy")) return 0;
@@ -411,10 +459,9 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_mesoscale_advance(long long key, int step
     }
     const Transport t = derive(c->config);
     cudaStream_t s = current_stream();
-    for (int k = 0; k < steps; ++k) {
-        const bool ok = c->hydro ? hydro_step(*c, t, c->fslot, c->fslot, s) : model_step(*c, t, c->fslot, s);
-        if (!ok) return 0;
-    }
+    if (!c->hydro) return model_steps(*c, t, c->fslot, steps, s) ? 1 : 0;
+    for (int k = 0; k < steps; ++k)
+        if (!hydro_step(*c, t, c->fslot, c->fslot, s)) return 0;
     return 1;
 }
 
