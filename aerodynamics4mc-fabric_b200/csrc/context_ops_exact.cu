@@ -153,9 +153,8 @@ __global__ void gather_temperature_kernel(const float* __restrict__ t, const uin
                                           int nz, OutBox b, float* __restrict__ out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.count()) return;
-    const int az = (int)(i % b.sz);
-    const int ay = (int)((i / b.sz) % b.sy);
-    const int ax = (int)(i / ((long long)b.sy * b.sz));
+    int ax, ay, az;
+    b.place(i, ax, ay, az);
     const int x = min(nx - 1, b.ox + ax * b.stride), y = min(ny - 1, b.oy + ay * b.stride),
               z = min(nz - 1, b.oz + az * b.stride);
     const long long cell = ((long long)x * ny + y) * nz + z;

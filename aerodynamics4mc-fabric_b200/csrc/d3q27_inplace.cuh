@@ -788,17 +788,14 @@ __global__ void output_ip_kernel(const typename S::T* __restrict__ f, IpArgs a, 
     const PadGeom G = a.g;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.count()) return;
-    const int az = (int)(i % b.sz);
-    const int ay = (int)((i / b.sz) % b.sy);
-    const int ax = (int)(i / ((long long)b.sy * b.sz));
+    int ax, ay, az;
+    b.place(i, ax, ay, az);
     const int x = min(G.nx - 1, b.ox + ax * b.stride), y = min(G.ny - 1, b.oy + ay * b.stride),
               z = min(G.nz - 1, b.oz + az * b.stride);
     const long long cell = ((long long)x * G.ny + y) * G.nz + z;
     float o4[4];
     macro_ip_cell<S, kExact>(f, a, G, cell, x, y, z, scale, o4);
-    float* dst = out + i * out_ch;
-    dst[0] = o4[0]; dst[1] = o4[1]; dst[2] = o4[2]; dst[3] = o4[3];
-    for (int c = 4; c < out_ch; ++c) dst[c] = 0.0f;
+    put_macro(out, i, out_ch, o4);
 }
 
 }  // namespace aero

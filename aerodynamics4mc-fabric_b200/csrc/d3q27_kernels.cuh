@@ -156,7 +156,32 @@ struct OutBox {
     int sx, sy, sz;
     int stride;
     __host__ __device__ long long count() const { return (long long)sx * sy * sz; }
+    // Place of output cell i; 32-bit divides where the count allows them.
+    __device__ __forceinline__ void place(long long i, int& ax, int& ay, int& az) const {
+        if (count() < (1LL << 32)) {
+            const unsigned c = (unsigned)i, row = c / (unsigned)sz;
+            az = (int)(c - row * (unsigned)sz);
+            ax = (int)(row / (unsigned)sy);
+            ay = (int)(row - (unsigned)ax * (unsigned)sy);
+        } else {
+            const long long row = i / sz;
+            az = (int)(i - row * sz);
+            ax = (int)(row / sy);
+            ay = (int)(row - (long long)ax * sy);
+        }
+    }
 };
+// Four macro values and the zeros up to the channel count; one 16-byte store
+// where the buffer allows it.
+__device__ __forceinline__ void put_macro(float* __restrict__ out, long long i, int out_ch, const float (&o)[4]) {
+    float* dst = out + i * out_ch;
+    if (out_ch == 4 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+        *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+        return;
+    }
+    dst[0] = o[0]; dst[1] = o[1]; dst[2] = o[2]; dst[3] = o[3];
+    for (int c = 4; c < out_ch; ++c) dst[c] = 0.0f;
+}
 inline OutBox strided_box(int nx, int ny, int nz, int stride) {
     return OutBox{0, 0, 0, (nx + stride - 1) / stride, (ny + stride - 1) / stride, (nz + stride - 1) / stride, stride};
 }

@@ -347,9 +347,8 @@ __global__ void output_ab_kernel(int nx, int ny, int nz, const float* __restrict
                                  float* __restrict__ out, int direct) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.count()) return;
-    const int az = (int)(i % b.sz);
-    const int ay = (int)((i / b.sz) % b.sy);
-    const int ax = (int)(i / ((long long)b.sy * b.sz));
+    int ax, ay, az;
+    b.place(i, ax, ay, az);
     const int x = min(nx - 1, b.ox + ax * b.stride), y = min(ny - 1, b.oy + ay * b.stride),
               z = min(nz - 1, b.oz + az * b.stride);
     const long long cells = (long long)nx * ny * nz;
@@ -366,9 +365,7 @@ __global__ void output_ab_kernel(int nx, int ny, int nz, const float* __restrict
     float o[4];
     if (kExact) exact::macro_out_exact(f, (w & kFlagSelfSolid) != 0, scale, o);
     else macro_out(f, (w & kFlagSelfSolid) != 0, scale, o);
-    float* dst = out + i * out_ch;
-    dst[0] = o[0]; dst[1] = o[1]; dst[2] = o[2]; dst[3] = o[3];
-    for (int c = 4; c < out_ch; ++c) dst[c] = 0.0f;
+    put_macro(out, i, out_ch, o);
 }
 
 template <bool kExact>

@@ -330,6 +330,68 @@ __device__ __forceinline__ void pull_model(const MesoArgs& A, long long i, int x
     }
 }
 
+// The same for the hydrodynamic distribution alone, in any storage, with the
+// wind from the forcing itself.
+template <class S, class I>
+__device__ __forceinline__ void pull_hydro(const HydroArgs& A, const typename S::T* __restrict__ src, long long i, uint32_t w,
+                                           float (&f)[19]) {
+    if (w & kHydroSelfSolid) {
+#pragma unroll
+        for (int q = 0; q < 19; ++q) f[q] = hfeq(q, 1.0f, 0.0f, 0.0f, 0.0f);
+        return;
+    }
+    const int nx = A.nx, ny = A.ny, nz = A.nz;
+    const I cells = (I)nx * (I)ny * (I)nz, own = (I)i;
+    int x, y, z;
+    cell_xyz32(i, ny, nz, x, y, z);
+    I X[3], Y[3], Z[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int sx = x + k - 1, sy = y + k - 1, sz = z + k - 1;
+        X[k] = (I)(sx < 0 ? sx + nx : (sx >= nx ? sx - nx : sx)) * ((I)ny * (I)nz);
+        Y[k] = (I)min(max(sy, 0), ny - 1) * (I)nz;
+        Z[k] = (I)(sz < 0 ? sz + nz : (sz >= nz ? sz - nz : sz));
+    }
+    const uint32_t ground = y == 0 ? mdirs(1, 1) : 0u;
+    const bool lid = A.free_slip_top && y == ny - 1;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) {
+        const I from = X[1 - mcx(q)] + Y[1 - mcy(q)] + Z[1 - mcz(q)] + (mcy(q) == -1 && lid ? (I)mmirror(q) : (I)q) * cells;
+        f[q] = S::load(src + (((w >> q) & 1u) ? (I)mopp(q) * cells + own : from), q, A.inv_scale);
+    }
+    if (!(w & kHydroSlow)) return;
+    uint32_t away = 0;
+    if (!A.periodic_sides)
+        away = (x == 0 ? mdirs(0, 1) : 0u) | (x == nx - 1 ? mdirs(0, -1) : 0u) | (z == 0 ? mdirs(2, 1) : 0u) |
+               (z == nz - 1 ? mdirs(2, -1) : 0u);
+    if (!A.free_slip_top && y == ny - 1) away |= mdirs(1, -1);
+    away &= ~ground;
+    int edge = min(min(x, z), min(nx - 1 - x, nz - 1 - z));
+    int top = ny - 1 - y;
+    if (A.periodic_sides) edge = 1 << 20;
+    if (A.free_slip_top) top = 1 << 20;
+    const int sponge = min(edge, top);
+    float alpha = sponge <= 0 ? 1.0f : (sponge < 2 ? 0.5f : 0.0f);
+    if (!A.edge_blend) alpha = 0.0f;
+    // the inflow wind is read only where a pull leaves the grid through an
+    // open side or the open top, or where the edge blend acts
+    if (away == 0 && alpha <= 0.0f) return;
+    const float* F = A.forcing_prev;
+    const float den = smax(1.0e-6f, A.velocity_scale);
+    const float bx = clamp_speed((ch(F, i, kChBackgroundWindX) + ch(F, i, kChNestedWindXDelta) + ch(F, i, kChConvectiveInflowX) +
+                                  ch(F, i, kChTornadoWindX)) / den);
+    const float bz = clamp_speed((ch(F, i, kChBackgroundWindZ) + ch(F, i, kChNestedWindZDelta) + ch(F, i, kChConvectiveInflowZ) +
+                                  ch(F, i, kChTornadoWindZ)) / den);
+    const float by = clamp_speed((ch(F, i, kChNestedUpdraft) + ch(F, i, kChTornadoUpdraft)) / den);
+#pragma unroll
+    for (int q = 0; q < 19; ++q) {
+        if (((w >> q) & 1u) && !((away >> q) & 1u)) continue;
+        const float fb = hfeq(q, 1.0f, bx, by, bz);
+        if ((away >> q) & 1u) f[q] = fb;
+        if (alpha > 0.0f) f[q] = (1.0f - alpha) * f[q] + alpha * fb;
+    }
+}
+
 // Targets + TRT of both distributions (native/src/aero_lbm_mesoscale.cpp:573-618).
 // kPull: the last step's streaming on the way in, so that a window of steps
 // reads and writes the populations once per step instead of twice
@@ -492,102 +554,28 @@ __global__ void meso_seed_kernel(MesoArgs A) {
 // seeded state; outputs stream the current post-collision state once more.
 // Two population buffers; each holds post-collision values.
 
-template <class S, int kMode>
+template <class S, int kMode, class I>
 __global__ void __launch_bounds__(256) meso_hydro_kernel(HydroArgs A) {
     using T = typename S::T;
     const int nx = A.nx, ny = A.ny, nz = A.nz;
-    const long long cells = (long long)nx * ny * nz;
+    const I cells = (I)nx * (I)ny * (I)nz;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cells) return;
-    int x, y, z;
-    cell_xyz32(i, ny, nz, x, y, z);
+    if (i >= (long long)nx * ny * nz) return;
+    const I own = (I)i;
     const T* __restrict__ src = static_cast<const T*>(A.src);
     float f[19];
     if (kMode == kHydroInit) {
 #pragma unroll
-        for (int q = 0; q < 19; ++q) f[q] = S::load(src + q * cells + i, q, A.inv_scale);
-    } else if (A.flags_prev[i] & kHydroSelfSolid) {
-#pragma unroll
-        for (int q = 0; q < 19; ++q) f[q] = hfeq(q, 1.0f, 0.0f, 0.0f, 0.0f);
-    } else if (!(A.flags_prev[i] & kHydroSlow)) {
-        // interior (or periodic / ground) cell: every source is known from the
-        // classification word, so the 19 loads are independent of each other
-        const uint32_t w = A.flags_prev[i];
-        long long idx[19];
-#pragma unroll
-        for (int q = 0; q < 19; ++q) {
-            int sx = x - mcx(q), sz = z - mcz(q);
-            if (A.periodic_sides) {
-                sx = sx < 0 ? sx + nx : (sx >= nx ? sx - nx : sx);
-                sz = sz < 0 ? sz + nz : (sz >= nz ? sz - nz : sz);
-            }
-            idx[q] = ((w >> q) & 1u) ? (long long)mopp(q) * cells + i : (long long)q * cells + midx(A, sx, y - mcy(q), sz);
-        }
-#pragma unroll
-        for (int q = 0; q < 19; ++q) f[q] = S::load(src + idx[q], q, A.inv_scale);
+        for (int q = 0; q < 19; ++q) f[q] = S::load(src + ((I)q * cells + own), q, A.inv_scale);
     } else {
-        int edge = min(min(x, z), min(nx - 1 - x, nz - 1 - z));
-        int top = ny - 1 - y;
-        if (A.periodic_sides) edge = 1 << 20;
-        if (A.free_slip_top) top = 1 << 20;
-        const int sponge = min(edge, top);
-        float alpha = sponge <= 0 ? 1.0f : (sponge < 2 ? 0.5f : 0.0f);
-        if (!A.edge_blend) alpha = 0.0f;
-        // the inflow wind is read only where a pull can leave the grid through
-        // an open side or the open top, or where the edge blend acts
-        float bx = 0.0f, by = 0.0f, bz = 0.0f;
-        if (alpha > 0.0f || edge <= 0 || top <= 0) {
-            const float* F = A.forcing_prev;
-            const float den = smax(1.0e-6f, A.velocity_scale);
-            bx = clamp_speed((ch(F, i, kChBackgroundWindX) + ch(F, i, kChNestedWindXDelta) + ch(F, i, kChConvectiveInflowX) +
-                              ch(F, i, kChTornadoWindX)) / den);
-            bz = clamp_speed((ch(F, i, kChBackgroundWindZ) + ch(F, i, kChNestedWindZDelta) + ch(F, i, kChConvectiveInflowZ) +
-                              ch(F, i, kChTornadoWindZ)) / den);
-            by = clamp_speed((ch(F, i, kChNestedUpdraft) + ch(F, i, kChTornadoUpdraft)) / den);
-        }
-#pragma unroll
-        for (int q = 0; q < 19; ++q) {
-            int sx = x - mcx(q), sy = y - mcy(q), sz = z - mcz(q);
-            if (A.periodic_sides) {
-                sx = sx < 0 ? sx + nx : (sx >= nx ? sx - nx : sx);
-                sz = sz < 0 ? sz + nz : (sz >= nz ? sz - nz : sz);
-            }
-            float fv;
-            bool bounced = false;
-            if (sx >= 0 && sx < nx && sy >= 0 && sy < ny && sz >= 0 && sz < nz) {
-                const long long sc = midx(A, sx, sy, sz);
-                if (A.solid_prev[sc]) {
-                    fv = S::load(src + mopp(q) * cells + i, mopp(q), A.inv_scale);
-                    bounced = true;
-                } else {
-                    fv = S::load(src + q * cells + sc, q, A.inv_scale);
-                }
-            } else if (sy < 0) {
-                fv = S::load(src + mopp(q) * cells + i, mopp(q), A.inv_scale);
-                bounced = true;
-            } else if (A.free_slip_top && sy >= ny && sx >= 0 && sx < nx && sz >= 0 && sz < nz) {
-                const long long sc = midx(A, sx, ny - 1, sz);
-                if (A.solid_prev[sc]) {
-                    fv = S::load(src + mopp(q) * cells + i, mopp(q), A.inv_scale);
-                    bounced = true;
-                } else {
-                    fv = S::load(src + mmirror(q) * cells + sc, mmirror(q), A.inv_scale);
-                }
-            } else {
-                fv = hfeq(q, 1.0f, bx, by, bz);
-            }
-            if (alpha > 0.0f && !bounced) {
-                const float fb = hfeq(q, 1.0f, bx, by, bz);
-                fv = (1.0f - alpha) * fv + alpha * fb;
-            }
-            f[q] = fv;
-        }
+        pull_hydro<S, I>(A, src, i, A.flags_prev[i], f);
     }
     if (kMode == kHydroOutput) {
-        float* o = A.out_state + i * kMesoStateChannels;
+        static_assert(kMesoStateChannels == 6, "three words of two floats");
+        float2* o = reinterpret_cast<float2*>(A.out_state) + 3 * i;
         if (A.flags_prev[i] & kHydroSelfSolid) {
-            o[0] = 1.0f;
-            o[1] = o[2] = o[3] = o[4] = o[5] = 0.0f;
+            o[0] = make_float2(1.0f, 0.0f);
+            o[1] = o[2] = make_float2(0.0f, 0.0f);
             return;
         }
         float r = 0.0f, ux = 0.0f, uy = 0.0f, uz = 0.0f;
@@ -603,12 +591,9 @@ __global__ void __launch_bounds__(256) meso_hydro_kernel(HydroArgs A) {
         uy /= r;
         uz /= r;
         const float ms = A.max_speed;
-        o[0] = r;
-        o[1] = 0.0f;
-        o[2] = 0.0f;
-        o[3] = sclamp(ux * A.velocity_scale, -ms, ms);
-        o[4] = sclamp(uy * A.velocity_scale, -ms, ms);
-        o[5] = sclamp(uz * A.velocity_scale, -ms, ms);
+        o[0] = make_float2(r, 0.0f);
+        o[1] = make_float2(0.0f, sclamp(ux * A.velocity_scale, -ms, ms));
+        o[2] = make_float2(sclamp(uy * A.velocity_scale, -ms, ms), sclamp(uz * A.velocity_scale, -ms, ms));
         return;
     }
     const bool solid = A.solid_cur[i] != 0;
@@ -631,7 +616,7 @@ __global__ void __launch_bounds__(256) meso_hydro_kernel(HydroArgs A) {
     trt_hydro(A.h, f, r, ux, uy, uz, solid, pf);
     T* __restrict__ dst = static_cast<T*>(A.dst);
 #pragma unroll
-    for (int q = 0; q < 19; ++q) S::store(dst + q * cells + i, q, pf[q], A.scale);
+    for (int q = 0; q < 19; ++q) S::store(dst + ((I)q * cells + own), q, pf[q], A.scale);
 }
 
 // Seed of the hydrodynamic-only state: seed_mesoscale_state's populations
@@ -777,14 +762,21 @@ cudaError_t meso_hydro_mask(const float* forcing, long long cells, uint8_t* soli
     return cudaGetLastError();
 }
 
-template <class S>
+template <class S, class I>
 static void hydro_dispatch(const meso::HydroArgs& a, int mode, unsigned blocks, int threads, cudaStream_t s) {
     if (mode == kHydroInit)
-        meso::meso_hydro_kernel<S, kHydroInit><<<blocks, threads, 0, s>>>(a);
+        meso::meso_hydro_kernel<S, kHydroInit, I><<<blocks, threads, 0, s>>>(a);
     else if (mode == kHydroStep)
-        meso::meso_hydro_kernel<S, kHydroStep><<<blocks, threads, 0, s>>>(a);
+        meso::meso_hydro_kernel<S, kHydroStep, I><<<blocks, threads, 0, s>>>(a);
     else
-        meso::meso_hydro_kernel<S, kHydroOutput><<<blocks, threads, 0, s>>>(a);
+        meso::meso_hydro_kernel<S, kHydroOutput, I><<<blocks, threads, 0, s>>>(a);
+}
+
+template <class S>
+static void hydro_dispatch(const meso::HydroArgs& a, int mode, unsigned blocks, int threads, cudaStream_t s) {
+    // 32-bit element indices where 19 x cells fits them
+    if (19LL * a.nx * a.ny * a.nz < (1LL << 32)) hydro_dispatch<S, unsigned>(a, mode, blocks, threads, s);
+    else hydro_dispatch<S, long long>(a, mode, blocks, threads, s);
 }
 
 cudaError_t meso_hydro_launch(const meso::HydroArgs& a, int mode, int storage, int threads, cudaStream_t s) {
