@@ -70,7 +70,7 @@ struct MesoArgs {
     const float* forcing;  // cells x 25 (AoS, as passed by the caller): seed and derivation only
     float* derived;        // kDCount x cells
     uint8_t* solid;
-    const uint32_t* flags; // pull classification (meso_hydro_flags)
+    uint32_t* flags;       // pull classification (meso_hydro_flags)
     const float* src_f;    // streamed, or (fused step, stream, ambient) post-collision populations
     const float* src_g;
     float* dst_f;
@@ -103,7 +103,7 @@ struct HydroArgs {
 }  // namespace meso
 
 cudaError_t meso_launch_seed(const meso::MesoArgs& a, cudaStream_t s);
-// Derived forcing and solid mask of a call's forcing.
+// Derived forcing, solid mask and pull classification of a call's forcing.
 cudaError_t meso_launch_derive(const meso::MesoArgs& a, cudaStream_t s);
 // Targets + TRT of the streamed state src into post-collision dst; pull: src
 // holds the last step's post-collision populations, streamed on the way in.

@@ -28,6 +28,7 @@
 #include "lattice.cuh"
 #include "meso.cuh"
 #include "meso_lattice.cuh"
+#include "pdl.cuh"
 
 namespace aero {
 namespace meso {
@@ -84,10 +85,55 @@ __device__ __forceinline__ float dv(const MesoArgs& A, int k, long long i) {
     return __ldg(A.derived + k * ((long long)A.nx * A.ny * A.nz) + i);
 }
 
+// Directions whose component along an axis is +1 / -1, as a bit set.
+__host__ __device__ constexpr uint32_t mdirs(int axis, int sign) {
+    uint32_t m = 0;
+    for (int q = 0; q < 19; ++q)
+        if ((axis == 0 ? mcx(q) : (axis == 1 ? mcy(q) : mcz(q))) == sign) m |= 1u << q;
+    return m;
+}
+
+// Pull classification of a fluid cell (see meso_hydro_flags): solid(n) of the
+// 19 sources is read whatever the cell's place (an open side's from the
+// wrapped cell, the ground's and the lid's from the cell's own row), so the
+// loads do not wait for one another.
+template <class Args, class Solid>
+__device__ __forceinline__ uint32_t pull_class(const Args& A, int x, int y, int z, Solid solid) {
+    const int nx = A.nx, ny = A.ny, nz = A.nz;
+    long long X[3], Y[3], Z[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int sx = x + k - 1, sy = y + k - 1, sz = z + k - 1;
+        X[k] = (long long)(sx < 0 ? sx + nx : (sx >= nx ? sx - nx : sx)) * ny * nz;
+        Y[k] = (long long)min(max(sy, 0), ny - 1) * nz;
+        Z[k] = sz < 0 ? sz + nz : (sz >= nz ? sz - nz : sz);
+    }
+    uint32_t hit = 0;
+#pragma unroll
+    for (int q = 0; q < 19; ++q)
+        hit |= solid(X[1 - mcx(q)] + Y[1 - mcy(q)] + Z[1 - mcz(q)]) ? 1u << q : 0u;
+    uint32_t side = 0;
+    if (!A.periodic_sides)
+        side = (x == 0 ? mdirs(0, 1) : 0u) | (x == nx - 1 ? mdirs(0, -1) : 0u) | (z == 0 ? mdirs(2, 1) : 0u) |
+               (z == nz - 1 ? mdirs(2, -1) : 0u);
+    const uint32_t ground = y == 0 ? mdirs(1, 1) : 0u, lid = y == ny - 1 ? mdirs(1, -1) : 0u;
+    // inside the grid (or reflected at a free-slip lid): off the solid cell
+    // there; the ground always; an open side or lid never
+    const uint32_t open = (side | (A.free_slip_top ? 0u : lid)) & ~ground;
+    const uint32_t w = (hit & ~open) | ground;
+    int edge = min(min(x, z), min(nx - 1 - x, nz - 1 - z));
+    int top = ny - 1 - y;
+    if (A.periodic_sides) edge = 1 << 20;
+    if (A.free_slip_top) top = 1 << 20;
+    const bool slow = (A.edge_blend && min(edge, top) < 2) || ((side | lid) & ~ground) != 0;
+    return w | (slow ? kHydroSlow : 0u);
+}
+
 // The forcing terms of compute_cell_targets and of the open boundaries that
 // do not depend on the state (native/src/aero_lbm_mesoscale.cpp:393-530,
 // 620-734), each expression as the reference has it.
 __global__ void __launch_bounds__(128) meso_derive_kernel(MesoArgs A) {
+    pdl_trigger();
     const long long cells = (long long)A.nx * A.ny * A.nz;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= cells) return;
@@ -119,7 +165,9 @@ __global__ void __launch_bounds__(128) meso_derive_kernel(MesoArgs A) {
     v[kDTornadoHeat] = ch(F, i, kChTornadoHeating);
     v[kDTornadoUp] = tor_up;
     v[kDNestedUp] = nest_up;
-    A.solid[i] = solid_at(F, i) ? 1 : 0;
+    const bool solid = solid_at(F, i);
+    A.solid[i] = solid ? 1 : 0;
+    A.flags[i] = solid ? kHydroSelfSolid : pull_class(A, x, y, z, [&](long long n) { return solid_at(F, n); });
 #pragma unroll
     for (int k = 0; k < kDCount; ++k) A.derived[k * cells + i] = v[k];
 }
@@ -242,14 +290,6 @@ __device__ __forceinline__ void trt_hydro(const HydroRates& H, const float (&f)[
         pf[q] = fep + fop + sq;
         pf[qo] = fep - fop + sqo;
     }
-}
-
-// Directions whose component along an axis is +1 / -1, as a bit set.
-__host__ __device__ constexpr uint32_t mdirs(int axis, int sign) {
-    uint32_t m = 0;
-    for (int q = 0; q < 19; ++q)
-        if ((axis == 0 ? mcx(q) : (axis == 1 ? mcy(q) : mcz(q))) == sign) m |= 1u << q;
-    return m;
 }
 
 // Streamed populations of cell i from the post-collision ones (pull
@@ -399,6 +439,8 @@ __device__ __forceinline__ void pull_hydro(const HydroArgs& A, const typename S:
 // stream over the forcing records).
 template <bool kPull, class I>
 __global__ void __launch_bounds__(128) meso_collide_kernel(MesoArgs A) {
+    pdl_trigger();
+    pdl_wait();
     const long long cells = (long long)A.nx * A.ny * A.nz;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= cells) return;
@@ -444,6 +486,8 @@ __global__ void __launch_bounds__(128) meso_collide_kernel(MesoArgs A) {
 
 template <class I>
 __global__ void __launch_bounds__(128) meso_ambient_kernel(MesoArgs A) {
+    pdl_trigger();
+    pdl_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)A.nx * A.ny * A.nz) return;
     int x, y, z;
@@ -464,6 +508,8 @@ __global__ void __launch_bounds__(128) meso_ambient_kernel(MesoArgs A) {
 // Pull streaming and macro export (native/src/aero_lbm_mesoscale.cpp:620-734).
 template <class I>
 __global__ void __launch_bounds__(128) meso_stream_kernel(MesoArgs A) {
+    pdl_trigger();
+    pdl_wait();
     const long long cells = (long long)A.nx * A.ny * A.nz;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= cells) return;
@@ -640,48 +686,12 @@ __global__ void meso_hydro_seed_kernel(const float* __restrict__ F, int nx, int 
     for (int q = 0; q < 19; ++q) S::store(dst + q * cells + i, q, hfeq(q, 1.0f, lx, ly, lz), scale);
 }
 
-// Pull classification of a mask (see meso_hydro_flags): the 19 mask bytes are
-// loaded whatever the cell's place (an open side's from the wrapped cell, the
-// ground's and the lid's from the cell's own row), so they do not wait for
-// one another.
 __global__ void meso_hydro_flags_kernel(HydroArgs A, const uint8_t* __restrict__ solid, uint32_t* __restrict__ flags) {
-    const int nx = A.nx, ny = A.ny, nz = A.nz;
-    const long long cells = (long long)nx * ny * nz;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cells) return;
-    if (solid[i]) {
-        flags[i] = kHydroSelfSolid;
-        return;
-    }
+    if (i >= (long long)A.nx * A.ny * A.nz) return;
     int x, y, z;
-    cell_xyz32(i, ny, nz, x, y, z);
-    long long X[3], Y[3], Z[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int sx = x + k - 1, sy = y + k - 1, sz = z + k - 1;
-        X[k] = (long long)(sx < 0 ? sx + nx : (sx >= nx ? sx - nx : sx)) * ny * nz;
-        Y[k] = (long long)min(max(sy, 0), ny - 1) * nz;
-        Z[k] = sz < 0 ? sz + nz : (sz >= nz ? sz - nz : sz);
-    }
-    uint32_t hit = 0;
-#pragma unroll
-    for (int q = 0; q < 19; ++q)
-        hit |= __ldg(solid + X[1 - mcx(q)] + Y[1 - mcy(q)] + Z[1 - mcz(q)]) ? 1u << q : 0u;
-    uint32_t side = 0;
-    if (!A.periodic_sides)
-        side = (x == 0 ? mdirs(0, 1) : 0u) | (x == nx - 1 ? mdirs(0, -1) : 0u) | (z == 0 ? mdirs(2, 1) : 0u) |
-               (z == nz - 1 ? mdirs(2, -1) : 0u);
-    const uint32_t ground = y == 0 ? mdirs(1, 1) : 0u, lid = y == ny - 1 ? mdirs(1, -1) : 0u;
-    // inside the grid (or reflected at a free-slip lid): off the solid cell
-    // there; the ground always; an open side or lid never
-    const uint32_t open = (side | (A.free_slip_top ? 0u : lid)) & ~ground;
-    const uint32_t w = (hit & ~open) | ground;
-    int edge = min(min(x, z), min(nx - 1 - x, nz - 1 - z));
-    int top = ny - 1 - y;
-    if (A.periodic_sides) edge = 1 << 20;
-    if (A.free_slip_top) top = 1 << 20;
-    const bool slow = (A.edge_blend && min(edge, top) < 2) || ((side | lid) & ~ground) != 0;
-    flags[i] = w | (slow ? kHydroSlow : 0u);
+    cell_xyz32(i, A.ny, A.nz, x, y, z);
+    flags[i] = solid[i] ? kHydroSelfSolid : pull_class(A, x, y, z, [&](long long n) { return __ldg(solid + n) != 0; });
 }
 
 __global__ void meso_mask_kernel(const float* __restrict__ F, long long cells, uint8_t* __restrict__ solid) {
@@ -709,27 +719,32 @@ cudaError_t meso_launch_derive(const meso::MesoArgs& a, cudaStream_t s) {
 // 32-bit population indices where they fit.
 static bool model_narrow(const meso::MesoArgs& a) { return 19LL * a.nx * a.ny * a.nz < (1LL << 32); }
 
+// The kernels of a step follow one another through programmatic launches:
+// each waits for its predecessor before it reads anything, so only the launch
+// gaps overlap (8 x 4 x 8 host-driven step 43.8 us against
+// 46.1 us one after the other, 42.0 with the classification in the derive
+// kernel; 128 x 24 x 128, 30 resident steps 2,036 against 2,160).
+template <class K>
+static cudaError_t model_launch(K kernel, const meso::MesoArgs& a, cudaStream_t s) {
+    count_launch();
+    return launch_pdl(kernel, dim3(model_blocks(a)), dim3(128), 0, s, a);
+}
+
 cudaError_t meso_launch_collide(const meso::MesoArgs& a, bool pull, cudaStream_t s) {
     using Wide = unsigned long long;
-    if (!pull) meso::meso_collide_kernel<false, Wide><<<model_blocks(a), 128, 0, s>>>(a);
-    else if (model_narrow(a)) meso::meso_collide_kernel<true, unsigned><<<model_blocks(a), 128, 0, s>>>(a);
-    else meso::meso_collide_kernel<true, Wide><<<model_blocks(a), 128, 0, s>>>(a);
-    count_launch();
-    return cudaGetLastError();
+    if (!pull) return model_launch(meso::meso_collide_kernel<false, Wide>, a, s);
+    return model_narrow(a) ? model_launch(meso::meso_collide_kernel<true, unsigned>, a, s)
+                           : model_launch(meso::meso_collide_kernel<true, Wide>, a, s);
 }
 
 cudaError_t meso_launch_ambient(const meso::MesoArgs& a, cudaStream_t s) {
-    if (model_narrow(a)) meso::meso_ambient_kernel<unsigned><<<model_blocks(a), 128, 0, s>>>(a);
-    else meso::meso_ambient_kernel<unsigned long long><<<model_blocks(a), 128, 0, s>>>(a);
-    count_launch();
-    return cudaGetLastError();
+    return model_narrow(a) ? model_launch(meso::meso_ambient_kernel<unsigned>, a, s)
+                           : model_launch(meso::meso_ambient_kernel<unsigned long long>, a, s);
 }
 
 cudaError_t meso_launch_stream(const meso::MesoArgs& a, cudaStream_t s) {
-    if (model_narrow(a)) meso::meso_stream_kernel<unsigned><<<model_blocks(a), 128, 0, s>>>(a);
-    else meso::meso_stream_kernel<unsigned long long><<<model_blocks(a), 128, 0, s>>>(a);
-    count_launch();
-    return cudaGetLastError();
+    return model_narrow(a) ? model_launch(meso::meso_stream_kernel<unsigned>, a, s)
+                           : model_launch(meso::meso_stream_kernel<unsigned long long>, a, s);
 }
 
 cudaError_t meso_hydro_seed(const float* forcing, int nx, int ny, int nz, float velocity_scale, int storage, float scale,

@@ -80,10 +80,10 @@ struct MesoContext {
 
     ~MesoContext() { release(); }
     void release() {
-        for (void* p : {(void*)forcing[0], (void*)forcing[1], (void*)solid[0], (void*)solid[1], (void*)flags[0],
-                        (void*)flags[1], (void*)f, (void*)g,
-                        (void*)pf, (void*)pg, (void*)derived, (void*)ambient, (void*)deep, (void*)surface, (void*)ndeep, (void*)nsurf,
-                        pop[0], pop[1], (void*)out})
+        // the model's flags and fields lie in the block of `derived`
+        for (void* p : {(void*)forcing[0], (void*)forcing[1], (void*)solid[0], (void*)solid[1],
+                        derived ? nullptr : (void*)flags[0], (void*)flags[1], (void*)f, (void*)g, (void*)pf, (void*)pg,
+                        (void*)derived, pop[0], pop[1], (void*)out})
             if (p) cudaFree(p);
         forcing[0] = forcing[1] = nullptr;
         solid[0] = solid[1] = nullptr;
@@ -119,20 +119,26 @@ bool allocate(MesoContext& c) {
     c.storage = c.hydro ? c.opt.storage : 0;
     const size_t n = (size_t)c.cells;
     bool ok = dev_alloc(&c.forcing[0], n * kMesoForcingChannels, "meso forcing") &&
-              dev_alloc(&c.forcing[1], n * kMesoForcingChannels, "meso forcing") &&
-              dev_alloc(&c.solid[0], n, "meso mask") && dev_alloc(&c.solid[1], n, "meso mask") &&
-              dev_alloc(&c.out, n * kMesoStateChannels, "meso output");
+              dev_alloc(&c.solid[0], n, "meso mask") && dev_alloc(&c.out, n * kMesoStateChannels, "meso output");
     if (!ok) return false;
     if (c.hydro) {
         const size_t bytes = n * 19 * (c.storage ? 2 : 4);
-        ok = cuda_ok(cudaMalloc(&c.pop[0], bytes), "meso populations") && cuda_ok(cudaMalloc(&c.pop[1], bytes), "meso populations") &&
+        ok = dev_alloc(&c.forcing[1], n * kMesoForcingChannels, "meso forcing") && dev_alloc(&c.solid[1], n, "meso mask") &&
+             cuda_ok(cudaMalloc(&c.pop[0], bytes), "meso populations") && cuda_ok(cudaMalloc(&c.pop[1], bytes), "meso populations") &&
              dev_alloc(&c.flags[0], n, "meso flags") && dev_alloc(&c.flags[1], n, "meso flags");
     } else {
-        ok = dev_alloc(&c.derived, n * meso::kDCount, "meso derived forcing") && dev_alloc(&c.flags[0], n, "meso flags") &&
-             dev_alloc(&c.f, n * 19, "meso f") && dev_alloc(&c.g, n * 19, "meso g") && dev_alloc(&c.pf, n * 19, "meso post f") &&
-             dev_alloc(&c.pg, n * 19, "meso post g") && dev_alloc(&c.ambient, n, "meso ambient") &&
-             dev_alloc(&c.deep, n, "meso deep") && dev_alloc(&c.surface, n, "meso surface") &&
-             dev_alloc(&c.ndeep, n, "meso deep") && dev_alloc(&c.nsurf, n, "meso surface");
+        // one forcing slot (read while the step that brings it is prepared);
+        // the per-cell planes in one block, c.derived holds it
+        ok = dev_alloc(&c.derived, n * (meso::kDCount + 6), "meso planes") && dev_alloc(&c.f, n * 19, "meso f") &&
+             dev_alloc(&c.g, n * 19, "meso g") && dev_alloc(&c.pf, n * 19, "meso post f") && dev_alloc(&c.pg, n * 19, "meso post g");
+        if (ok) {
+            float* plane = c.derived + n * meso::kDCount;
+            for (float** p : {&c.ambient, &c.deep, &c.surface, &c.ndeep, &c.nsurf}) {
+                *p = plane;
+                plane += n;
+            }
+            c.flags[0] = reinterpret_cast<uint32_t*>(plane);
+        }
     }
     return ok;
 }
@@ -207,15 +213,7 @@ int hydro_threads(const MesoContext& c) { return c.opt.threads > 0 ? c.opt.threa
 
 // The derived forcing, mask and pull classification of forcing slot `slot`.
 bool model_inputs(MesoContext& c, const Transport& t, int slot, cudaStream_t s) {
-    meso::HydroArgs h = {};
-    h.nx = c.nx;
-    h.ny = c.ny;
-    h.nz = c.nz;
-    h.periodic_sides = c.opt.periodic_sides ? 1 : 0;
-    h.free_slip_top = c.opt.free_slip_top ? 1 : 0;
-    h.edge_blend = c.opt.disable_edge_blend ? 0 : 1;
-    return cuda_ok(meso_launch_derive(model_args(c, t, slot, nullptr), s), "mesoscale forcing") &&
-           cuda_ok(meso_hydro_flags(h, c.solid[0], c.flags[0], s), "mesoscale flags");
+    return cuda_ok(meso_launch_derive(model_args(c, t, slot, nullptr), s), "mesoscale forcing");
 }
 
 // `steps` steps of the reference model on forcing slot `slot`: collide the
@@ -363,7 +361,7 @@ AERO_LBM_B200_EXPORT int aero_lbm_mesoscale_step_context(long long key, const Ae
     const Transport t = derive(*config);
     cudaStream_t s = current_stream();
     const size_t fbytes = (size_t)c->cells * kMesoForcingChannels * sizeof(float);
-    const int slot = c->initialized ? (c->fslot ^ 1) : 0;
+    const int slot = c->hydro && c->initialized ? (c->fslot ^ 1) : 0;
     if (!cuda_ok(cudaMemcpyAsync(c->forcing[slot], forcing, fbytes, cudaMemcpyHostToDevice, s), "mesoscale forcing upload"))
         return 0;
     if (c->hydro) {
