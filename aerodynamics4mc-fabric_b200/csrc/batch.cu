@@ -383,7 +383,7 @@ struct Batch {
     int class_begin[kBrickClasses + 1] = {};  // first unit of each class
     int* d_publish_brick = nullptr;
     int publish_blocks = 0;
-    float* d_flow = nullptr;       // copy_flow's device output, one largest brick, allocated at the first copy
+    float* d_flow = nullptr;       // copy_flow's device output, one largest brick
     short* d_atlas = nullptr;
     int atlas_records = 0;
     int stride = 4;
@@ -531,6 +531,14 @@ bool build_units(Batch& B, int threads) {
     B.atlas_records = atlas;
     B.shape.threads = threads;
     return true;
+}
+
+cudaError_t alloc_flow(Batch& B) {
+    size_t most = 0;
+    for (const HostBrick& k : B.bricks) most = std::max(most, (size_t)k.nx * k.ny * k.nz);
+    const cudaError_t e = cudaMalloc(&B.d_flow, most * 4 * sizeof(float));
+    if (e != cudaSuccess) B.d_flow = nullptr;
+    return e;
 }
 
 // A tick's first class starts when all before it has completed. The later
@@ -785,6 +793,7 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_batch_finalize(long long handle, int publ
     if (!bok(cudaMemsetAsync(B->d_atlas, 0, (size_t)atlas * 4 * sizeof(short), s), "memset(atlas)")) return 0;
     if (!bok(cudaStreamSynchronize(s), "sync")) return 0;
     if (!build_units(*B, B->shape.threads)) return 0;
+    if (alloc_flow(*B) != cudaSuccess) cudaGetLastError();  // copy_flow asks again
     B->bytes_per_tick = bytes;
     B->finalized = true;
     // host copies are not needed any more
@@ -933,14 +942,7 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_batch_copy_flow(long long handle, int bri
         return 0;
     }
     cudaStream_t s = current_stream();
-    if (!B->d_flow) {
-        size_t most = 0;
-        for (const HostBrick& k : B->bricks) most = std::max(most, (size_t)k.nx * k.ny * k.nz);
-        if (!bok(cudaMalloc(&B->d_flow, most * 4 * sizeof(float)), "cudaMalloc(flow)")) {
-            B->d_flow = nullptr;
-            return 0;
-        }
-    }
+    if (!B->d_flow && !bok(alloc_flow(*B), "cudaMalloc(flow)")) return 0;
     batch_flow_kernel<<<(cells + 127) / 128, 128, 0, s>>>(B->d_descs, brick, B->parity, B->d_flow);
     count_launch();
     const bool ok = bok(cudaGetLastError(), "batch_flow_kernel") &&
