@@ -590,7 +590,7 @@ class LbmContext:
 
 
 class BrickBatch:
-    """Batched bricks advanced by one persistent launch per tick
+    """Batched bricks advanced by one launch per tick and class of bricks
     (aero_lbm_b200_batch_*)."""
 
     def __init__(self, lib: ctypes.CDLL | None = None):

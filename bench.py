@@ -350,7 +350,7 @@ def run_batch_leg(aero, lib, torch, stream, ticks: int, warmup: int) -> dict:
     """C4: 400 x 32^3 + 80 x 64^3 + 32 x 128^3 bricks (seeded masks with solid
     fraction U[0, 0.15], tau U[0.51, 0.6], body force U[-1e-5, 1e-5]^3),
     alternating FP32 / FP16 storage, periodic x/y and bounce-back z faces, one
-    persistent launch + stride-4 int16 publish per tick, graph replay,
+    launch per storage + stride-4 int16 publish per tick, graph replay,
     autotuned launch shape."""
     rng = np.random.default_rng(4)
     b = aero.BrickBatch(lib)

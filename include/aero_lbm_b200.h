@@ -359,8 +359,9 @@ AERO_LBM_B200_EXPORT void aero_lbm_b200_set_physics_overrides(float smagorinsky_
 /* ---- batched bricks (no reference counterpart: the reference steps bricks one
  * aero_lbm_step_rect call at a time, native/src/aero_lbm_simulation_bridge.cpp:1092-1166) ----
  * Many independent bricks of uneven sizes, each with its own mask, relaxation
- * time, body force and storage precision, advanced by one persistent launch
- * per tick, with a stride-s packed int16 velocity publish per tick. */
+ * time, body force and storage precision, advanced by one launch per class
+ * (storage, parity of nz) and tick, with a stride-s packed int16 velocity
+ * publish per tick. */
 AERO_LBM_B200_EXPORT int aero_lbm_b200_batch_create(long long* out_handle);
 /* precision 0 = fp32, 1 = fp16 deviation storage; obstacle: cells bytes (or
  * null); init_velocity_soa: 3 x cells floats (or null = rest); tau in
