@@ -69,13 +69,13 @@ __device__ __forceinline__ long long midx(const Args& A, int x, int y, int z) {
 }
 // horizontal (x, z) and vertical (y) laplacians with clamped neighbours
 // (native/src/aero_lbm_mesoscale.cpp:335-373)
-__device__ __forceinline__ float hlap(const MesoArgs& A, const float* __restrict__ a, int x, int y, int z) {
+__device__ __forceinline__ float hlap(const MesoArgs& A, const float* a, int x, int y, int z) {
     const float c = a[midx(A, x, y, z)];
     const float xp = a[midx(A, min(A.nx - 1, x + 1), y, z)], xm = a[midx(A, max(0, x - 1), y, z)];
     const float zp = a[midx(A, x, y, min(A.nz - 1, z + 1))], zm = a[midx(A, x, y, max(0, z - 1))];
     return xp + xm + zp + zm - 4.0f * c;
 }
-__device__ __forceinline__ float vlap(const MesoArgs& A, const float* __restrict__ a, int x, int y, int z) {
+__device__ __forceinline__ float vlap(const MesoArgs& A, const float* a, int x, int y, int z) {
     if (A.ny <= 1) return 0.0f;
     const float c = a[midx(A, x, y, z)];
     const float yp = a[midx(A, x, min(A.ny - 1, y + 1), z)], ym = a[midx(A, x, max(0, y - 1), z)];
@@ -83,7 +83,7 @@ __device__ __forceinline__ float vlap(const MesoArgs& A, const float* __restrict
 }
 
 __device__ __forceinline__ float dv(const MesoArgs& A, int k, long long i) {
-    return __ldg(A.derived + k * ((long long)A.nx * A.ny * A.nz) + i);
+    return A.derived[k * ((long long)A.nx * A.ny * A.nz) + i];
 }
 
 // Directions whose component along an axis is +1 / -1, as a bit set.
@@ -177,15 +177,16 @@ struct Targets {
     float rho, ux, uy, uz, teq, nsurf, ndeep;
 };
 
-// compute_cell_targets (native/src/aero_lbm_mesoscale.cpp:393-530)
+// compute_cell_targets (native/src/aero_lbm_mesoscale.cpp:393-530); D: the
+// cell's derived forcing terms
 __device__ __forceinline__ Targets cell_targets(const MesoArgs& A, const float (&f)[19], const float (&g)[19], long long i,
-                                                int x, int y, int z, bool solid) {
+                                                int x, int y, int z, bool solid, const float (&D)[kDCount]) {
     const float dt = smax(1.0e-3f, A.dt_s);
     const float amb_relax = sclamp(dt / 600.0f, 0.0f, 1.0f);
     const float deep_relax = sclamp(dt / 2400.0f, 0.0f, 1.0f);
     const float surf_relax = sclamp(dt / 300.0f, 0.0f, 1.0f);
     const float wind_relax = sclamp(dt / 60.0f, 0.0f, 1.0f);
-    const float deep_t = dv(A, kDDeep, i), surf_t = dv(A, kDSurface, i);
+    const float deep_t = D[kDDeep], surf_t = D[kDSurface];
     if (solid) return Targets{1.0f, 0.0f, 0.0f, 0.0f, surf_t, surf_t, deep_t};
     float r = 0.0f, ux = 0.0f, uy = 0.0f, uz = 0.0f, amb = 0.0f;
 #pragma unroll
@@ -200,11 +201,11 @@ __device__ __forceinline__ Targets cell_targets(const MesoArgs& A, const float (
     ux /= r;
     uy /= r;
     uz /= r;
-    const float amb_t = dv(A, kDAmbient, i);
-    const float conv_h = dv(A, kDConvHeat, i), tor_h = dv(A, kDTornadoHeat, i);
-    const float tor_up = dv(A, kDTornadoUp, i), nest_up = dv(A, kDNestedUp, i);
-    const float hum = dv(A, kDHumidity, i);
-    const float sx = dv(A, kDSlopeX, i), sz = dv(A, kDSlopeZ, i);
+    const float amb_t = D[kDAmbient];
+    const float conv_h = D[kDConvHeat], tor_h = D[kDTornadoHeat];
+    const float tor_up = D[kDTornadoUp], nest_up = D[kDNestedUp];
+    const float hum = D[kDHumidity];
+    const float sx = D[kDSlopeX], sz = D[kDSlopeZ];
     const float s_hl = hlap(A, A.surface, x, y, z), s_vl = vlap(A, A.surface, x, y, z);
     const float d_vl = vlap(A, A.deep, x, y, z);
     const float a_hl = hlap(A, A.ambient, x, y, z), a_vl = vlap(A, A.ambient, x, y, z);
@@ -213,14 +214,14 @@ __device__ __forceinline__ Targets cell_targets(const MesoArgs& A, const float (
     const float damp = 1.0f - 0.12f * hum;
     const float nsurf = surf_i + surf_relax * damp * (surf_t - surf_i) + 0.10f * (ndeep - surf_i) + 0.04f * conv_h +
                         0.08f * tor_h + 0.05f * s_hl + 0.025f * s_vl;
-    const float lx = dv(A, kDLatticeX, i), ly = dv(A, kDLatticeY, i), lz = dv(A, kDLatticeZ, i);
+    const float lx = D[kDLatticeX], ly = D[kDLatticeY], lz = D[kDLatticeZ];
     const float push = 0.0008f * (nsurf - amb);
     const float nsw = 1.0f - (float)y / smax(1.0f, (float)(A.ny - 1));
     const float lift = 0.0015f * (lx * sx + lz * sz) * nsw;
     const float blift = 0.0009f * (nsurf - amb) * nsw;
     const float steer_x = -0.005f * sx * lz;
     const float steer_z = 0.005f * sz * lx;
-    const float drag = dv(A, kDDrag, i);
+    const float drag = D[kDDrag];
     const float tux = clamp_speed(lx + steer_x + push * sx - drag * ux);
     const float tuz = clamp_speed(lz + steer_z + push * sz - drag * uz);
     const float tuy = clamp_speed(ly + lift + blift - drag * uy);
@@ -306,11 +307,9 @@ __device__ __forceinline__ void pull_model(const MesoArgs& A, long long i, int x
                                            float (&gn)[19]) {
     const int nx = A.nx, ny = A.ny, nz = A.nz;
     const I cells = (I)nx * (I)ny * (I)nz, own = (I)i;
-    const float* __restrict__ pf = A.src_f;
-    const float* __restrict__ pg = A.src_g;
-    const float* __restrict__ wall = A.derived + kDSurface * (long long)cells;
+    const float *pf = A.src_f, *pg = A.src_g, *wall = A.derived + kDSurface * (long long)cells;
     if (w & kHydroSelfSolid) {
-        const float wt = __ldg(wall + i);
+        const float wt = wall[i];
 #pragma unroll
         for (int q = 0; q < 19; ++q) {
             if (kHydro) fn[q] = hfeq(q, 1.0f, 0.0f, 0.0f, 0.0f);
@@ -335,8 +334,8 @@ __device__ __forceinline__ void pull_model(const MesoArgs& A, long long i, int x
         const I src = ((ground >> q) & 1u) ? own : X[1 - mcx(q)] + Y[1 - mcy(q)] + Z[1 - mcz(q)];
         // specular reflection at the lid: the mirrored population of the same row
         const I from = (mcy(q) == -1 && (lid >> q) & 1u) ? (I)mmirror(q) * cells + src : (I)q * cells + src;
-        if (kHydro) fn[q] = __ldg(pf + (bounced ? (I)mopp(q) * cells + own : from));
-        gn[q] = __ldg(bounced ? wall + src : pg + from);
+        if (kHydro) fn[q] = pf[bounced ? (I)mopp(q) * cells + own : from];
+        gn[q] = *(bounced ? wall + src : pg + from);
     }
 #pragma unroll
     for (int q = 0; q < 19; ++q)
@@ -448,6 +447,12 @@ __global__ void __launch_bounds__(128) meso_collide_kernel(MesoArgs A) {
     int x, y, z;
     cell_xyz32(i, A.ny, A.nz, x, y, z);
     const uint32_t w = A.flags[i];
+    // the derived terms first: ordinary loads (pdl.cuh) that no branch or store
+    // of the pull holds back (128 x 24 x 128, 30 steps: 1,963 us against 2,081
+    // where cell_targets loads them)
+    float D[kDCount];
+#pragma unroll
+    for (int k = 0; k < kDCount; ++k) D[k] = dv(A, k, i);
     float f[19], g[19];
     if (kPull) {
         pull_model<true, I>(A, i, x, y, z, w, f, g);
@@ -459,7 +464,7 @@ __global__ void __launch_bounds__(128) meso_collide_kernel(MesoArgs A) {
         }
     }
     const bool solid = (w & kHydroSelfSolid) != 0;
-    const Targets t = cell_targets(A, f, g, i, x, y, z, solid);
+    const Targets t = cell_targets(A, f, g, i, x, y, z, solid, D);
     A.next_deep[i] = t.ndeep;
     A.next_surface[i] = t.nsurf;
     float pf[19];
@@ -728,7 +733,7 @@ static bool model_narrow(const meso::MesoArgs& a) { return 19LL * a.nx * a.ny * 
 // each waits for its predecessor before it reads anything, so only the launch
 // gaps overlap (8 x 4 x 8 host-driven step 43.8 us against
 // 46.1 us one after the other, 42.0 with the classification in the derive
-// kernel; 128 x 24 x 128, 30 resident steps 2,036 against 2,160).
+// kernel; 128 x 24 x 128, 30 resident steps 2,081 against 2,161).
 template <class K>
 static cudaError_t model_launch(K kernel, const meso::MesoArgs& a, cudaStream_t s) {
     count_launch();

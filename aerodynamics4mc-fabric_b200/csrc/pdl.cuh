@@ -2,7 +2,11 @@
 // kernel launched with launch_pdl may be scheduled while its predecessor on
 // the stream still runs. It must call pdl_wait() before it reads anything the
 // predecessor writes; the wait returns once the predecessor grid has
-// completed and its memory operations are visible. pdl_trigger() at the top
+// completed and its memory operations are visible. After it, what an earlier
+// kernel wrote is read by ordinary loads: __ldg, or a const __restrict__
+// pointer that lets the compiler choose the same load, promises data that is
+// constant from this kernel's start, which lies before the predecessor's end,
+// and the wait need not order such a load. pdl_trigger() at the top
 // of a kernel lets its own dependent be scheduled once every block of this
 // grid has started (the dependent's blocks then hold their slots and wait).
 // Without the launch attribute, or after a predecessor that never triggers,
