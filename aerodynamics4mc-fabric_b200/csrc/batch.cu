@@ -216,7 +216,7 @@ __device__ __forceinline__ void stage_step(BrickStep& sd, const BrickDesc& d, in
 // shared memory, with the slots' offsets worked out by the host.
 template <class S, bool kPairs, int kParity>
 __global__ void __maxnreg__(kPairs ? 96 : 80)
-    batch_step_kernel(const BrickDesc* __restrict__ descs, const int* __restrict__ unit_brick, int begin, int end) {
+    batch_step_kernel(const BrickDesc* descs, const int* unit_brick, int begin, int end) {
     __shared__ BrickStep sd;
     pdl_trigger();
     for (int u = begin + (int)blockIdx.x; u < end; u += gridDim.x) {

@@ -286,14 +286,14 @@ struct PairIO;
 template <>
 struct PairIO<StoreF32> {
     __device__ __forceinline__ static F2 load(const float* p0, const float* p1, int, const Fp16Scale&) {
-        return f2(__ldg(p0), __ldg(p1));
+        return f2(*p0, *p1);
     }
     __device__ __forceinline__ static F2 load2(const float* p, int, const Fp16Scale&) {
-        return F2{__ldg(reinterpret_cast<const float2*>(p))};
+        return F2{*reinterpret_cast<const float2*>(p)};
     }
     __device__ __forceinline__ static F2 load2p(const float* p, const float* p1, bool fix, int, const Fp16Scale&) {
-        float2 r = __ldg(reinterpret_cast<const float2*>(p));
-        if (fix) r.y = __ldg(p1);
+        float2 r = *reinterpret_cast<const float2*>(p);
+        if (fix) r.y = *p1;
         return F2{r};
     }
     __device__ __forceinline__ static F2 unscaled(F2 v, float by) { return by == 1.0f ? v : f2(by) * v; }
@@ -317,15 +317,15 @@ struct PairIO<StoreF16Dev> {
         return __ffma2_rn(v.v, make_float2(k, k), make_float2(-s.scale, -s.scale));
     }
     __device__ __forceinline__ static F2 load(const __half* p0, const __half* p1, int q, const Fp16Scale& s) {
-        return decode(make_float2(__half2float(__ldg(p0)), __half2float(__ldg(p1))), q, s);
+        return decode(make_float2(__half2float(*p0), __half2float(*p1)), q, s);
     }
     __device__ __forceinline__ static F2 load2(const __half* p, int q, const Fp16Scale& s) {
-        return decode(__half22float2(__ldg(reinterpret_cast<const __half2*>(p))), q, s);
+        return decode(__half22float2(*reinterpret_cast<const __half2*>(p)), q, s);
     }
     __device__ __forceinline__ static F2 load2p(const __half* p, const __half* p1, bool fix, int q, const Fp16Scale& s) {
-        const __half2 r = __ldg(reinterpret_cast<const __half2*>(p));
+        const __half2 r = *reinterpret_cast<const __half2*>(p);
         __half y = __high2half(r);
-        if (fix) y = __ldg(p1);
+        if (fix) y = *p1;
         return decode(make_float2(__low2float(r), __half2float(y)), q, s);
     }
     __device__ __forceinline__ static void store(__half* p0, __half* p1, bool s0, bool s1, int q, F2 v, const Fp16Scale& s, float by = 1.0f) {
@@ -350,15 +350,15 @@ struct PairIO<StoreI16Dev> {
         return __ffma2_rn(v.v, make_float2(k, k), make_float2(-s.scale, -s.scale));
     }
     __device__ __forceinline__ static F2 load(const short* p0, const short* p1, int q, const Fp16Scale& s) {
-        const unsigned r = (unsigned)(unsigned short)__ldg(p0) | ((unsigned)(unsigned short)__ldg(p1) << 16);
+        const unsigned r = (unsigned)(unsigned short)*p0 | ((unsigned)(unsigned short)*p1 << 16);
         return decode(s16x2_to_float2(r), q, s);
     }
     __device__ __forceinline__ static F2 load2(const short* p, int q, const Fp16Scale& s) {
-        return decode(s16x2_to_float2(__ldg(reinterpret_cast<const unsigned*>(p))), q, s);
+        return decode(s16x2_to_float2(*reinterpret_cast<const unsigned*>(p)), q, s);
     }
     __device__ __forceinline__ static F2 load2p(const short* p, const short* p1, bool fix, int q, const Fp16Scale& s) {
-        unsigned r = __ldg(reinterpret_cast<const unsigned*>(p));
-        if (fix) r = (r & 0xFFFFu) | ((unsigned)(unsigned short)__ldg(p1) << 16);
+        unsigned r = *reinterpret_cast<const unsigned*>(p);
+        if (fix) r = (r & 0xFFFFu) | ((unsigned)(unsigned short)*p1 << 16);
         return decode(s16x2_to_float2(r), q, s);
     }
     __device__ __forceinline__ static void store(short* p0, short* p1, bool s0, bool s1, int q, F2 v, const Fp16Scale& s, float by = 1.0f) {
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(128, kExact ? AERO_IP2X_MIN_BLOCKS : AERO_IP2_
 // bounce-back value in the cell's flipped slot of parity p. Products and sums
 // round separately (the reference's order).
 template <class S>
-__device__ __forceinline__ float ip_face_source(const typename S::T* __restrict__ f, const IpArgs& a, const PadGeom& G,
+__device__ __forceinline__ float ip_face_source(const typename S::T* f, const IpArgs& a, const PadGeom& G,
                                                 const NeighbourOffsets& o, int own, long long cell, int x, int y, int z,
                                                 int q, int sx, int sy, int sz, int p) {
     const FaceParams& F = *a.face_prev;

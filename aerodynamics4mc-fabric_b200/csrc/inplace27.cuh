@@ -40,12 +40,14 @@ struct Fp16Scale {
     float inv_scale;  // 1 / S
 };
 
-// Population storage policies.
+// Population storage policies. Loads are ordinary ones: the step writes the
+// slots that it reads, and may start before the kernel in front has ended
+// (pdl.cuh).
 struct StoreF32 {
     using T = float;
-    __device__ __forceinline__ static float load(const float* __restrict__ a, int q, const Fp16Scale&) {
+    __device__ __forceinline__ static float load(const float* a, int q, const Fp16Scale&) {
         (void)q;
-        return __ldg(a);
+        return *a;
     }
     __device__ __forceinline__ static void store(float* __restrict__ a, int q, float v, const Fp16Scale&) {
         (void)q;
@@ -60,8 +62,8 @@ struct StoreF32 {
 // reference's rule for non-finite populations).
 struct StoreF16Dev {
     using T = __half;
-    __device__ __forceinline__ static float load(const __half* __restrict__ a, int q, const Fp16Scale& s) {
-        const float h = __half2float(__ldg(a));
+    __device__ __forceinline__ static float load(const __half* a, int q, const Fp16Scale& s) {
+        const float h = __half2float(*a);
         return fmaf(h, q_w(q) * s.inv_scale, q_w(q));
     }
     __device__ __forceinline__ static void store(__half* __restrict__ a, int q, float v, const Fp16Scale& s) {
@@ -96,8 +98,8 @@ __device__ __forceinline__ float2 s16x2_to_float2(unsigned w) {
 }
 struct StoreI16Dev {
     using T = short;
-    __device__ __forceinline__ static float load(const short* __restrict__ a, int q, const Fp16Scale& s) {
-        return fmaf((float)__ldg(a), q_w(q) * s.inv_scale, q_w(q));
+    __device__ __forceinline__ static float load(const short* a, int q, const Fp16Scale& s) {
+        return fmaf((float)*a, q_w(q) * s.inv_scale, q_w(q));
     }
     __device__ __forceinline__ static void store(short* __restrict__ a, int q, float v, const Fp16Scale& s) {
         *a = sat_round_s16(fmaf(v, s.scale * (1.0f / q_w(q)), -s.scale));

@@ -395,8 +395,8 @@ __device__ __forceinline__ void fetch_plane(const ThermalArgs& a, const StageSlo
         if (gxe < 0 || !s.valid(e)) continue;
         if (s.vec(e)) {
             const int c = base + s.off[e];
-            const float2 t2 = __ldg(reinterpret_cast<const float2*>(a.t + c));
-            const unsigned short m2 = __ldg(reinterpret_cast<const unsigned short*>(a.obstacle + c));
+            const float2 t2 = *reinterpret_cast<const float2*>(a.t + c);
+            const unsigned short m2 = *reinterpret_cast<const unsigned short*>(a.obstacle + c);
             r.t[e][0] = t2.x;
             r.t[e][1] = t2.y;
             r.m |= (unsigned)m2 << (16 * e);
@@ -405,8 +405,8 @@ __device__ __forceinline__ void fetch_plane(const ThermalArgs& a, const StageSlo
             for (int k = 0; k < 2; ++k) {
                 const int o = src.off[s.idx[e] + k];
                 if (o >= 0) {
-                    r.m |= (unsigned)__ldg(a.obstacle + base + o) << (8 * (2 * e + k));
-                    r.t[e][k] = __ldg(a.t + base + o);
+                    r.m |= (unsigned)a.obstacle[base + o] << (8 * (2 * e + k));
+                    r.t[e][k] = a.t[base + o];
                 }
             }
         }

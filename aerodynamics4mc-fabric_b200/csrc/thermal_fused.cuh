@@ -76,7 +76,7 @@ __device__ __forceinline__ void stage_entry(const FusedTransport& tr, const uint
     }
     const long long cell = ((long long)x * ny + y) * nz + z;
     code = obstacle[cell] ? 1 : 0;
-    if (!code) v = __ldg(tr.t + cell);
+    if (!code) v = tr.t[cell];
 }
 
 // Stage the nine rows of a block's z-segment [z_begin, z_begin + span) plus a
@@ -111,7 +111,7 @@ __device__ __forceinline__ void stage_rows(const FusedTransport& tr, const uint8
             const float* t = tr.t + row;
             for (int k = 1 + threadIdx.x; k <= span; k += blockDim.x) {
                 const unsigned char code = ob[k] ? 1 : 0;
-                const float v = __ldg(t + k);
+                const float v = t[k];
                 put_entry<kTagged>(sv, sc, r * W + k, code ? 0.0f : v, code);
             }
         }
@@ -176,7 +176,7 @@ __device__ __forceinline__ float update(const FusedTransport& tr, const uint8_t*
     const int ctr = 4 * W + k;  // row (0, 0)
     const float tc = sv[ctr];
     const float ux = tr.u[cell], uy = tr.u[cell + (long long)nx * ny * nz], uz = tr.u[cell + 2LL * nx * ny * nz];
-    const float src = tr.source ? exact::rclamp(__ldg(tr.source + cell), -0.006f, 0.006f) : 0.0f;
+    const float src = tr.source ? exact::rclamp(tr.source[cell], -0.006f, 0.006f) : 0.0f;
     const float px = __fsub_rn((float)x, __fmul_rn(dt, ux));
     const float py = __fsub_rn((float)y, __fmul_rn(dt, uy));
     const float pz = __fsub_rn((float)z, __fmul_rn(dt, uz));

@@ -75,6 +75,10 @@ def waiting_kernels_reach(unit: str) -> dict[str, list[tuple[str, str]]]:
 
 @pytest.mark.parametrize("unit,kernels", [
     ("meso_exact.cu", {"meso_collide_kernel", "meso_ambient_kernel", "meso_stream_kernel"}),
+    ("d3q27_exact.cu", {"step_ip2_kernel"}),
+    ("d3q27_fast.cu", {"step_ip2_kernel"}),
+    ("thermal_exact.cu", {"thermal_update_kernel", "thermal_fill_kernel"}),
+    ("batch.cu", {"batch_step_kernel"}),
 ])
 def test_waiting_kernels_use_ordinary_loads(unit, kernels):
     reach = waiting_kernels_reach(unit)
