@@ -30,7 +30,7 @@ struct IpArgs {
     ForceField force;
     CollideParams cp;
     Fp16Scale sc;
-    int cells_per_thread;            // 1 one cell per thread, 2 two cells per thread (packed collision)
+    int cells_per_thread;            // 1 one cell per thread, 2 two cells per thread (packed collision), 0 by the brick's size
     int streamed;                    // factorised two-cell step: populations streamed by bulk async copies
     int* fault;                      // device word set to 1 by a streamed step whose copies never landed
     // Temperature transport computed by the step kernel itself (1) before each

@@ -44,11 +44,12 @@ struct IpLaunch {
         step_timer_begin(s);
         // the runtime terms (fans, state nudge, sponge) exist in the one-cell kernel only
         int cpt = a.cp.runtime_terms ? 1 : a.cells_per_thread;
-        // In the reference's order the two forms give the same bits, and a
-        // brick whose one-cell grid is a single wave is bound by one warp's
-        // latency, which the one-cell form has less of (32^3: 8.2 against 10.1
-        // us a step, 24^3 8.2 against 10.5; 40^3, two waves, 12.3 against 11.4).
-        if (kExact && cpt == 2 && !a.transport && one_wave(a.g)) cpt = 1;
+        // Without a form of the caller's choice: in the reference's order the
+        // two give the same bits, and a brick whose one-cell grid is a single
+        // wave is bound by one warp's latency, which the one-cell form has less
+        // of (32^3: 8.2 against 10.1 us a step, 24^3 8.2 against 10.5; 40^3,
+        // two waves, 12.3 against 11.4).
+        if (cpt == 0) cpt = kExact && !a.transport && one_wave(a.g) ? 1 : 2;
         if (!kExact && cpt == 2 && a.streamed && !a.transport && IpaLaunch<S>::eligible(a)) {
             cudaError_t e = IpaLaunch<S>::step(f, a, s);
             if (e != cudaSuccess) return e;

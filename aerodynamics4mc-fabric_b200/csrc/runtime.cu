@@ -64,7 +64,7 @@ void drop_pending_fill(Context& ctx) {
 int g_thermal_mode = -1;      // temperature transport: -1 with buoyancy, 0 never (packet field), 1 always
 int g_streamed_step = 0;      // factorised two-cell in-place step: bulk-copy streamed kernel where eligible (opt-in)
 int g_fused_transport = 0;    // in-place steps compute the first-order temperature transport themselves (opt-in)
-int g_cells_per_thread = 2;    // in-place step: 1 one cell per thread, 2 two cells per thread (packed collision)
+int g_cells_per_thread = 0;    // in-place step: 1 one cell per thread, 2 two cells per thread (packed collision), 0 by the brick's size
 int g_fp16_format = 1;         // 16-bit storage: 0 IEEE half deviations, 1 fixed-point deviations (default)
 std::unordered_map<long long, std::unique_ptr<Context>> g_contexts;
 std::string g_last_error;
@@ -2218,7 +2218,7 @@ AERO_LBM_B200_EXPORT void aero_lbm_b200_reset_tuning(void) {
     g_thermal_mode = -1;
     g_streamed_step = 0;
     g_fused_transport = 0;
-    g_cells_per_thread = 2;
+    g_cells_per_thread = 0;
     g_fp16_format = 1;
     g_stream_mode = 0;
     g_collision_mode = 0;

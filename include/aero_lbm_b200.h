@@ -312,9 +312,12 @@ AERO_LBM_B200_EXPORT int aero_lbm_b200_conservation_sums_noalloc(long long conte
  * agrees to FP32 rounding per step). */
 AERO_LBM_B200_EXPORT int aero_lbm_b200_set_collision_mode(int mode);
 /* Launch shape of the in-place step: 2 = two z-adjacent cells per thread with
- * the collision in sm_100 packed FP32 (default), 1 = one cell per thread. With
+ * the collision in sm_100 packed FP32, 1 = one cell per thread. With
  * the reference-order collision both shapes are bit-identical; with the
- * factorised one they agree to FP32 rounding. */
+ * factorised one they agree to FP32 rounding. Until it is called (and after
+ * aero_lbm_b200_reset_tuning) the library chooses: 2, but 1 for a
+ * reference-order brick whose one-cell grid fits the device at once (up to
+ * 34^3 on a B200). A brick in game-runtime mode always steps one cell per thread. */
 AERO_LBM_B200_EXPORT int aero_lbm_b200_set_cells_per_thread(int cells_per_thread);
 /* Temperature transport before every collision (the reference's
  * benchmark-mode update: first-order semi-Lagrangian advection by the
