@@ -780,34 +780,44 @@ bool steps_together(const World& w, const Brick& b) {
            !b.pending_reinit && b.stepped_context == b.context && b.stepped_version == b.static_version;
 }
 
+// Launches of at most kWorldChunk bricks; a launch that fails costs its own
+// bricks their contexts and no others.
 bool step_together(Service& svc, World& w, const std::vector<TogetherBrick>& bricks) {
     ModeScope scope(w.solver_mode);
-    const int n = w.brick_size;
-    std::vector<WorldStepJob> jobs;
-    jobs.reserve(bricks.size());
-    for (const TogetherBrick& t : bricks) {
-        w.packet_build_steps++;
-        w.d3q27_steps++;
-        t.brick->compact_active = false;
-        jobs.push_back(WorldStepJob{find_context(t.brick->context), fill_args(w, t.coord, *t.brick, t.brick->cur),
-                                    sync_args(svc, w, *t.brick, 1 - t.brick->cur, t.brick->cur)});
+    bool all_ok = true;
+    for (size_t at = 0; at < bricks.size(); at += kWorldChunk) {
+        const std::vector<TogetherBrick> group(bricks.begin() + at, bricks.begin() + std::min(bricks.size(), at + kWorldChunk));
+        std::vector<WorldStepJob> jobs;
+        jobs.reserve(group.size());
+        for (const TogetherBrick& t : group) {
+            w.packet_build_steps++;
+            w.d3q27_steps++;
+            t.brick->compact_active = false;
+            jobs.push_back(WorldStepJob{find_context(t.brick->context), fill_args(w, t.coord, *t.brick, t.brick->cur),
+                                        sync_args(svc, w, *t.brick, 1 - t.brick->cur, t.brick->cur)});
+        }
+        if (!world_step_batch(jobs)) {
+            set_sim_error("brick_step_actual: aero_lbm_step_rect failed at " + coord_text(group.front().coord) +
+                          (group.size() > 1 ? " to " + coord_text(group.back().coord) + " (" + std::to_string(group.size()) +
+                                                  " bricks stepped together)"
+                                            : std::string()) +
+                          ": " + last_error());
+            for (const TogetherBrick& t : group) release_context(svc, *t.brick);
+            all_ok = false;
+            continue;
+        }
+        for (const TogetherBrick& t : group) {
+            Brick& b = *t.brick;
+            b.cur = 1 - b.cur;
+            expect_flag(svc, b);
+            b.constrained_version = b.static_version;
+            b.stale = false;
+            update_shell(w, t.coord, b);
+            b.pending_patch_cells.clear();
+            b.pending_reinit = b.geometry_dirty = b.forcing_dirty = false;
+        }
     }
-    if (!world_step_batch(jobs)) {
-        set_sim_error("brick_step_actual: aero_lbm_step_rect failed at " + coord_text(bricks.front().coord) + ": " + last_error());
-        for (const TogetherBrick& t : bricks) release_context(svc, *t.brick);
-        return false;
-    }
-    for (const TogetherBrick& t : bricks) {
-        Brick& b = *t.brick;
-        b.cur = 1 - b.cur;
-        expect_flag(svc, b);
-        b.constrained_version = b.static_version;
-        b.stale = false;
-        update_shell(w, t.coord, b);
-        b.pending_patch_cells.clear();
-        b.pending_reinit = b.geometry_dirty = b.forcing_dirty = false;
-    }
-    return true;
+    return all_ok;
 }
 
 // step_brick_actual (simulation_bridge.cpp:1706-1832)
@@ -998,6 +1008,13 @@ bool step_world(Service& svc, long long wkey, World& w, int steps) {
         }
         std::vector<Fallback> fallbacks;
         std::vector<TogetherBrick> together;
+        // the tick ends early at a brick that fails: those in front of it step all the same
+        auto fail = [&] {
+            const std::string why = last_error();
+            if (!together.empty()) (void)step_together(svc, w, together);
+            set_error(why);
+            return false;
+        };
         SnapshotCache cache;
         for (auto& [c, b] : w.bricks) {
             if (!solver_active(w, b) || !b.has_dynamic) continue;
@@ -1007,7 +1024,7 @@ bool step_world(Service& svc, long long wkey, World& w, int steps) {
                 if (!step_brick(svc, w, c, b, next, fallbacks)) all_ok = false;
                 continue;
             }
-            if (!ensure_dynamic(svc, w, b) || !device_ready(svc, w, b)) return false;
+            if (!ensure_dynamic(svc, w, b) || !device_ready(svc, w, b)) return fail();
             if (!seed && steps_together(w, b) && world_step_ready(find_context(b.context), n, n, n)) {
                 together.push_back(TogetherBrick{c, &b});
                 continue;
@@ -1016,7 +1033,7 @@ bool step_world(Service& svc, long long wkey, World& w, int steps) {
             Next next{b.cur, nullptr, b.nonzero};
             if (seed || bootstrap) {
                 auto host = std::make_unique<HostDynamic>();
-                if (!pull(w, b, b.cur, *host)) return false;
+                if (!pull(w, b, b.cur, *host)) return fail();
                 bool seeded = !seed;
                 if (seed) {
                     // seed_brick_from_boundary_reference (simulation_bridge.cpp:1333-1348), then the neighbours' means
@@ -1037,7 +1054,7 @@ bool step_world(Service& svc, long long wkey, World& w, int steps) {
                 const bool nz = host_nonzero(*host);
                 if (seed && !seeded && !nz) continue;
                 host_constrain(*b.stat, *host);
-                if (!upload_dynamic(w, b, 1 - b.cur, *host)) return false;
+                if (!upload_dynamic(w, b, 1 - b.cur, *host)) return fail();
                 next.buffer = 1 - b.cur;
                 next.nonzero = host_nonzero(*host);
                 next.host = std::move(host);

@@ -8,6 +8,10 @@
 
 namespace aero {
 
+// Bricks one launch of a world's tick takes (their arguments travel in the
+// launch's parameter space, 32764 bytes at most).
+constexpr int kWorldChunk = 32;
+
 // Face configuration the pull of one step uses (a snapshot: the pull of call
 // n+1 streams with the faces of call n, as the reference streams at the end of
 // call n).

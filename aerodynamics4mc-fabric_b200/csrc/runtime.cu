@@ -1058,6 +1058,11 @@ bool world_step_ready(const Context* c, int nx, int ny, int nz) {
 // exchange before them and the refresh flags after them are the caller's).
 bool world_step_batch(const std::vector<WorldStepJob>& jobs) {
     if (jobs.empty()) return true;
+    const size_t n = jobs.size();
+    if (n > kWorldChunk) {
+        set_error("world step: too many bricks for one launch");
+        return false;
+    }
     const auto t0 = Clock::now();
     clear_error();
     cudaStream_t s = current_stream();
@@ -1065,64 +1070,61 @@ bool world_step_batch(const std::vector<WorldStepJob>& jobs) {
     CollideParams cp = current_collide_params();
     const bool thermal = g_thermal_mode == 1 || (g_thermal_mode == -1 && cp.enable_buoyancy);
     const unsigned fill_faces = fill_face_mask(face);
-    for (size_t at = 0; at < jobs.size(); at += kWorldChunk) {
-        const size_t n = std::min<size_t>(kWorldChunk, jobs.size() - at);
-        std::vector<WorldInputs> in(n);
-        std::vector<WorldStep> step[2], post(n);
-        std::vector<WorldOutput> out(n);
-        std::vector<ThermalArgs> heat;
-        for (size_t i = 0; i < n; ++i) {
-            const WorldStepJob& job = jobs[at + i];
-            Context& c = *job.ctx;
-            c.thermal = thermal;
-            cp.nx = c.nx;
-            cp.ny = c.ny;
-            cp.nz = c.nz;
-            cp.step = c.step_counter;
-            const int from = c.slot, to = 1 - c.slot;
-            in[i] = WorldInputs{job.fill, c.fields(to), ThermalNudgeArgs{}, job.sync.flag};
-            if (thermal) {
-                in[i].nudge = ThermalNudgeArgs{c.nx, c.ny, c.nz, c.temperature, c.obstacle[to], c.ref_temperature, cp.state_nudge};
-                if (c.step_counter % 2 == 0) {
-                    // runtime mode updates the temperature every other call (BFECC)
-                    heat.push_back(thermal_args(c, c.obstacle[to], cp));
-                    std::swap(c.temperature, c.temperature_scratch);
-                }
+    std::vector<WorldInputs> in(n);
+    std::vector<WorldStep> step[2], post(n);
+    std::vector<WorldOutput> out(n);
+    std::vector<ThermalArgs> heat;
+    for (size_t i = 0; i < n; ++i) {
+        const WorldStepJob& job = jobs[i];
+        Context& c = *job.ctx;
+        c.thermal = thermal;
+        cp.nx = c.nx;
+        cp.ny = c.ny;
+        cp.nz = c.nz;
+        cp.step = c.step_counter;
+        const int from = c.slot, to = 1 - c.slot;
+        in[i] = WorldInputs{job.fill, c.fields(to), ThermalNudgeArgs{}, job.sync.flag};
+        if (thermal) {
+            in[i].nudge = ThermalNudgeArgs{c.nx, c.ny, c.nz, c.temperature, c.obstacle[to], c.ref_temperature, cp.state_nudge};
+            if (c.step_counter % 2 == 0) {
+                // runtime mode updates the temperature every other call (BFECC)
+                heat.push_back(thermal_args(c, c.obstacle[to], cp));
+                std::swap(c.temperature, c.temperature_scratch);
             }
-            // the mask is unchanged: both slots hold (or now take) the same classification
-            if (!c.slots_match) {
-                if (!cuda_ok(cudaMemcpyAsync(c.d_face[to], c.d_face[from], sizeof(FaceParams), cudaMemcpyDeviceToDevice, s), "copy faces") ||
-                    !cuda_ok(cudaMemcpyAsync(c.flags[to], c.flags[from], (size_t)c.cells * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s),
-                             "copy classification"))
-                    return false;
-                c.slots_match = true;
-            }
-            c.h_face[to] = face;
-            WorldStep st{static_cast<float*>(c.ip), ip_args(c, from, to, cp)};
-            st.a.parity = c.parity;
-            step[c.parity & 1].push_back(st);
-            c.parity ^= 1;
-            st.a = ip_args(c, to, to, cp);
-            st.a.parity = c.parity;
-            st.a.fill_faces = fill_faces;
-            post[i] = st;
-            out[i] = WorldOutput{st.f, st.a, job.sync};
-            out[i].sync.temperature = c.temperature;
-            c.slot = to;
-            c.face_prev = face;
-            c.step_counter += 1;
-            c.force_valid = false;
         }
-        bool ok = cuda_ok(launch_world_inputs(in.data(), (int)n, s), "world inputs");
-        if (ok && !heat.empty()) ok = cuda_ok(launch_bfecc_batch(heat.data(), (int)heat.size(), s), "world temperature");
-        for (int p = 0; p < 2 && ok; ++p)
-            if (!step[p].empty()) ok = cuda_ok(launch_world_step(step[p].data(), (int)step[p].size(), p, s), "world step");
-        if (ok && fill_faces) ok = cuda_ok(launch_world_face_fill(post.data(), (int)n, s), "world face pre-fill");
-        if (ok) ok = cuda_ok(launch_world_output(out.data(), (int)n, s), "world output");
-        if (!ok) return false;
+        // the mask is unchanged: both slots hold (or now take) the same classification
+        if (!c.slots_match) {
+            if (!cuda_ok(cudaMemcpyAsync(c.d_face[to], c.d_face[from], sizeof(FaceParams), cudaMemcpyDeviceToDevice, s), "copy faces") ||
+                !cuda_ok(cudaMemcpyAsync(c.flags[to], c.flags[from], (size_t)c.cells * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s),
+                         "copy classification"))
+                return false;
+            c.slots_match = true;
+        }
+        c.h_face[to] = face;
+        WorldStep st{static_cast<float*>(c.ip), ip_args(c, from, to, cp)};
+        st.a.parity = c.parity;
+        step[c.parity & 1].push_back(st);
+        c.parity ^= 1;
+        st.a = ip_args(c, to, to, cp);
+        st.a.parity = c.parity;
+        st.a.fill_faces = fill_faces;
+        post[i] = st;
+        out[i] = WorldOutput{st.f, st.a, job.sync};
+        out[i].sync.temperature = c.temperature;
+        c.slot = to;
+        c.face_prev = face;
+        c.step_counter += 1;
+        c.force_valid = false;
     }
-    const double ms = ms_since(t0) / (double)jobs.size();
-    for (size_t i = 0; i < jobs.size(); ++i) record_timing(0.0, 0.0, 0.0, ms, false);
+    bool ok = cuda_ok(launch_world_inputs(in.data(), (int)n, s), "world inputs");
+    if (ok && !heat.empty()) ok = cuda_ok(launch_bfecc_batch(heat.data(), (int)heat.size(), s), "world temperature");
+    for (int p = 0; p < 2 && ok; ++p)
+        if (!step[p].empty()) ok = cuda_ok(launch_world_step(step[p].data(), (int)step[p].size(), p, s), "world step");
+    if (ok && fill_faces) ok = cuda_ok(launch_world_face_fill(post.data(), (int)n, s), "world face pre-fill");
+    if (ok) ok = cuda_ok(launch_world_output(out.data(), (int)n, s), "world output");
+    if (!ok) return false;
+    const double ms = ms_since(t0) / (double)n;
+    for (size_t i = 0; i < n; ++i) record_timing(0.0, 0.0, 0.0, ms, false);
     return true;
 }
 

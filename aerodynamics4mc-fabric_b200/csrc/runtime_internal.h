@@ -158,7 +158,8 @@ struct WorldStepJob {
 // in runtime mode, stepped before, with nothing staged or pending.
 bool world_step_ready(const Context* ctx, int nx, int ny, int nz);
 // The calls of step_rect_device (mask unchanged) and the flow output of each
-// job's context, launched over all jobs (one size) together.
+// job's context, launched over all jobs (one size, at most kWorldChunk of
+// them) together. After a failure the state of their contexts is lost.
 bool world_step_batch(const std::vector<WorldStepJob>& jobs);
 // A packed atlas straight from a context's populations; false in *done when
 // the context's layout has no such pass.

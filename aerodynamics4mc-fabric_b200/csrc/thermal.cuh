@@ -111,9 +111,6 @@ __device__ __forceinline__ void thermal_nudge_cell(const ThermalNudgeArgs& a, lo
     a.t[cell] = clamp1(a.t[cell] * keep + rt * n);
 }
 
-// Bricks one launch of a world's tick takes (their arguments travel in the
-// launch's parameter space, 32764 bytes at most).
-constexpr int kWorldChunk = 32;
 // The BFECC update of n <= kWorldChunk bricks of one size: three launches.
 cudaError_t launch_bfecc_batch(const ThermalArgs* args, int n, cudaStream_t s);
 
