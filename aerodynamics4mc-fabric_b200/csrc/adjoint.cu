@@ -309,11 +309,13 @@ __global__ void adj_seed_kernel(Geo G, const float* __restrict__ s, float ux_in,
 // registers allow. Of the block sizes that keep 20 warps, 320 threads measured
 // best where the grid fills the chip (64^3, sweep per call: 72 us against 74
 // of 128, 78 of 64 and 72 of 640 threads); below about one and a half waves
-// the smaller blocks spread better (48^3: 36.5 against 33.9 us, 56^3: 44.9
-// against 46.2), so rev_threads_for draws the line there.
+// the smaller blocks spread better (48^3: 36.5 us with 320 threads, 33.9 with
+// 128; 56^3: 44.9 and 46.2), so rev_threads_for draws the line there.
 constexpr int kRevThreads = 320, kRevThreadsSmall = 128;
-constexpr long long kRevWaveCells = 148LL * 2 * kRevThreads;
-int rev_threads_for(long long cells) { return 2 * cells >= 3 * kRevWaveCells ? kRevThreads : kRevThreadsSmall; }
+int rev_threads_for(long long cells) {
+    const long long wave = 2LL * kRevThreads * device_sms();
+    return 2 * cells >= 3 * wave ? kRevThreads : kRevThreadsSmall;
+}
 template <bool kInit, class I>
 __global__ void __launch_bounds__(kRevThreads, 2) adj_reverse_kernel(StepArgs<float> A, const float* __restrict__ lam_n,
                                                           float* __restrict__ lam_prev, double* __restrict__ grad_f,

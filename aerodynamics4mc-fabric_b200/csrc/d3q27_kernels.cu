@@ -20,6 +20,17 @@ std::atomic<uint64_t> g_launches{0};
 uint64_t kernel_launch_count() { return g_launches.load(); }
 void count_launch() { g_launches.fetch_add(1); }
 
+int device_sms() {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];  // per device, 0: not asked yet
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+    if (dev < kDevices && (sms = known[dev].load()) > 0) return sms;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 1;
+    if (dev < kDevices) known[dev].store(sms);
+    return sms;
+}
+
 namespace {
 struct StepTimer {
     bool on = false;

@@ -225,6 +225,8 @@ cudaError_t launch_output_ab_fast(BrickDims d, const float* g, const uint32_t* f
 
 uint64_t kernel_launch_count();
 void count_launch();
+// SMs of the current device.
+int device_sms();
 // Optional CUDA-event timing of the brick step kernel launches (off unless
 // aero_lbm_b200_kernel_timer enabled it): brackets one launch on stream s.
 void step_timer_begin(cudaStream_t s);

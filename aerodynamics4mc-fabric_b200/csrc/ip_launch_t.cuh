@@ -20,8 +20,8 @@ inline void fill_slot_offsets(IpArgs& a) {
 }
 
 // Whether the one-cell step's grid is at most one wave (4 blocks of 128
-// threads of its 128 registers on each of 148 SMs).
-inline bool one_wave(const PadGeom& g) { return (long long)g.nx * g.ny * ((g.nz + 31) / 32) * 32 <= 148LL * 512; }
+// threads of its 128 registers on each SM).
+inline bool one_wave(const PadGeom& g) { return (long long)g.nx * g.ny * ((g.nz + 31) / 32) * 32 <= 512LL * device_sms(); }
 
 template <class S, bool kExact>
 struct IpLaunch {
