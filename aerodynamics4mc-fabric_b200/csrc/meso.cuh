@@ -69,7 +69,6 @@ struct MesoArgs {
     float omega_t_even, omega_t_odd;
     const float* forcing;  // cells x 25 (AoS, as passed by the caller): seed and derivation only
     float* derived;        // kDCount x cells
-    uint8_t* solid;
     uint32_t* flags;       // pull classification (meso_hydro_flags)
     const float* src_f;    // streamed, or (fused step, stream, ambient) post-collision populations
     const float* src_g;
@@ -103,7 +102,7 @@ struct HydroArgs {
 }  // namespace meso
 
 cudaError_t meso_launch_seed(const meso::MesoArgs& a, cudaStream_t s);
-// Derived forcing, solid mask and pull classification of a call's forcing.
+// Derived forcing and pull classification of a call's forcing.
 cudaError_t meso_launch_derive(const meso::MesoArgs& a, cudaStream_t s);
 // Targets + TRT of the streamed state src into post-collision dst; pull: src
 // holds the last step's post-collision populations, streamed on the way in.

@@ -5,7 +5,7 @@
 // top, macro export (native/src/aero_lbm_mesoscale.cpp:146-738).
 //
 // A call from the host is three launches: `meso_derive_kernel` (what the step
-// reads of the forcing, the mask and the pull classification),
+// reads of the forcing and the pull classification),
 // `meso_collide_kernel` (targets + TRT, one thread per cell; writes post-collision f and g and the next surface /
 // deep-ground temperatures) and `meso_stream_kernel` (pull + boundaries +
 // macro export; writes the new f and g, the ambient field and the output
@@ -167,7 +167,6 @@ __global__ void __launch_bounds__(128) meso_derive_kernel(MesoArgs A) {
     v[kDTornadoUp] = tor_up;
     v[kDNestedUp] = nest_up;
     const bool solid = solid_at(F, i);
-    A.solid[i] = solid ? 1 : 0;
     A.flags[i] = solid ? kHydroSelfSolid : pull_class(A, x, y, z, [&](long long n) { return solid_at(F, n); });
 #pragma unroll
     for (int k = 0; k < kDCount; ++k) A.derived[k * cells + i] = v[k];

@@ -1,8 +1,9 @@
 // Host side of the D3Q19 mesoscale ABI: contexts keyed like the reference's
 // (native/src/aero_lbm_mesoscale.cpp:215-240, 1397-1510), per-call transport
-// derivation, seeding, and the two step paths: the reference model (two
+// derivation, seeding, and the two step paths: the reference model (three
 // launches per call, hydrodynamic + thermal distributions) and the
-// hydrodynamic-only fused step (one launch per call, FP32 or FP16 storage).
+// hydrodynamic-only fused step (one launch per call; FP32, FP16 or 16-bit
+// fixed-point storage).
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -65,8 +66,8 @@ struct MesoContext {
     int storage = 0;        // kMesoStore* of the allocated state (hydro only)
     float fp16_scale = 1.0f;
     float* forcing[2] = {nullptr, nullptr};
-    uint8_t* solid[2] = {nullptr, nullptr};
-    uint32_t* flags[2] = {nullptr, nullptr};  // hydro: pull classification of solid[k]
+    uint8_t* solid[2] = {nullptr, nullptr};   // hydro: masks (the model's is in its classification)
+    uint32_t* flags[2] = {nullptr, nullptr};  // pull classification (hydro: of solid[k])
     int fslot = 0;          // forcing / mask of the last step call
     // reference model
     float *f = nullptr, *g = nullptr, *pf = nullptr, *pg = nullptr;
@@ -76,7 +77,6 @@ struct MesoContext {
     void* pop[2] = {nullptr, nullptr};
     int cur = 0;
     float* out = nullptr;   // device output state, cells x 6
-    bool out_valid = false; // reference model: out holds the last step's state
 
     ~MesoContext() { release(); }
     void release() {
@@ -92,7 +92,6 @@ struct MesoContext {
         pop[0] = pop[1] = nullptr;
         cells = 0;
         initialized = false;
-        out_valid = false;
     }
     double bytes_per_step() const {
         if (hydro) return (double)cells * (19.0 * 2.0 * (storage ? 2.0 : 4.0) + 1.0);
@@ -119,11 +118,12 @@ bool allocate(MesoContext& c) {
     c.storage = c.hydro ? c.opt.storage : 0;
     const size_t n = (size_t)c.cells;
     bool ok = dev_alloc(&c.forcing[0], n * kMesoForcingChannels, "meso forcing") &&
-              dev_alloc(&c.solid[0], n, "meso mask") && dev_alloc(&c.out, n * kMesoStateChannels, "meso output");
+              dev_alloc(&c.out, n * kMesoStateChannels, "meso output");
     if (!ok) return false;
     if (c.hydro) {
         const size_t bytes = n * 19 * (c.storage ? 2 : 4);
-        ok = dev_alloc(&c.forcing[1], n * kMesoForcingChannels, "meso forcing") && dev_alloc(&c.solid[1], n, "meso mask") &&
+        ok = dev_alloc(&c.forcing[1], n * kMesoForcingChannels, "meso forcing") &&
+             dev_alloc(&c.solid[0], n, "meso mask") && dev_alloc(&c.solid[1], n, "meso mask") &&
              cuda_ok(cudaMalloc(&c.pop[0], bytes), "meso populations") && cuda_ok(cudaMalloc(&c.pop[1], bytes), "meso populations") &&
              dev_alloc(&c.flags[0], n, "meso flags") && dev_alloc(&c.flags[1], n, "meso flags");
     } else {
@@ -175,7 +175,6 @@ meso::MesoArgs model_args(MesoContext& c, const Transport& t, int slot, float* o
     a.omega_t_odd = 1.0f / trt_odd_tau(tau_t);
     a.forcing = c.forcing[slot];
     a.derived = c.derived;
-    a.solid = c.solid[0];
     a.flags = c.flags[0];
     a.ambient = c.ambient;
     a.deep = c.deep;
@@ -211,7 +210,7 @@ meso::HydroArgs hydro_args(const MesoContext& c, const Transport& t, int prev_sl
 
 int hydro_threads(const MesoContext& c) { return c.opt.threads > 0 ? c.opt.threads : 256; }
 
-// The derived forcing, mask and pull classification of forcing slot `slot`.
+// The derived forcing and pull classification of forcing slot `slot`.
 bool model_inputs(MesoContext& c, const Transport& t, int slot, cudaStream_t s) {
     return cuda_ok(meso_launch_derive(model_args(c, t, slot, nullptr), s), "mesoscale forcing");
 }
@@ -251,7 +250,6 @@ bool model_steps(MesoContext& c, const Transport& t, int slot, int steps, cudaSt
     a.dst_f = c.f;
     a.dst_g = c.g;
     if (!cuda_ok(meso_launch_stream(a, s), "mesoscale stream")) return false;
-    c.out_valid = true;
     return true;
 }
 
