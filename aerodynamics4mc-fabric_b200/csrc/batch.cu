@@ -269,7 +269,7 @@ __device__ __forceinline__ void publish_cell(const BrickDesc& b, int x, int y, i
 // publish_brick). Each record gathers 27 populations from as many cache
 // lines, so the launch needs every record in flight at once; one block per
 // brick, walking its records, took 166 us a tick for 24 bricks of 32^3 to
-// 96^3 (60 k records), against 12 us in this form.
+// 96^3 (60 k records), against 11 us in this form.
 constexpr int kPublishThreads = 128;
 __global__ void __launch_bounds__(kPublishThreads) batch_publish_kernel(const BrickDesc* __restrict__ descs,
                                                                         const int* __restrict__ publish_brick, int parity,

@@ -178,8 +178,8 @@ struct MesoPair<MesoI16> {
 // the launch-uniform offsets of a direction are 32-bit and every slot address
 // is the pair's own address plus one of them.
 //
-// Bound: issue and load latency, not memory (256 x 64 x 256: 356 MB a step in
-// 16 bits, 54 us at the measured copy rate). Every lane issues its 19 loads
+// Bound: issue and load latency, not memory (256 x 64 x 256: 340 MB a step in
+// 16 bits, classification and mask included, 52 us at the measured copy rate). Every lane issues its 19 loads
 // through one selected address each: no divergent slow pull, and the lid, the
 // ground and open sides ride along, so a warp at the lid keeps the uniform
 // path. Blocks per SM by storage: the 16-bit forms hold their raw words in
